@@ -311,3 +311,125 @@ def tolerance(case):
     1.9e-6.  The bf16 and fp16 figures are the rounding of P, dS and the results."""
     return {"bf16": {"rel": 1e-2, "max": 0.3}, "fp16": {"rel": 1.3e-3, "max": 2.2e-2},
             "fp32": {"rel": 1.7e-6, "max": 8e-6}}[case["dtype"]]
+
+
+# ---------------------------------------------------------------------------- the same in 64 bits
+def _attend(q, k, v, visible, scale, do=None):
+    """Softmax attention of q [T, G, D] over k, v [N, D] in float64, `visible(r0, r1)` being the
+    [1 or G, r1 - r0, N] mask of the rows: (o, natural-log lse), and with `do` also (dq, dk, dv)."""
+    t, g, d = q.shape
+    n = k.shape[0]
+    q, k, v = q.double().transpose(0, 1), k.double(), v.double()
+    o, lse = torch.empty_like(q), q.new_empty(g, t)
+    if do is not None:
+        do = do.double().transpose(0, 1)
+        dq, dk, dv = torch.empty_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    step = max(1, (1 << 26) // (g * n))
+    for r0 in range(0, t, step):
+        r1 = min(t, r0 + step)
+        s = (q[:, r0:r1] @ k.T).mul_(scale).masked_fill_(~visible(r0, r1), -math.inf)
+        lse[:, r0:r1] = s.logsumexp(-1)
+        p = s.sub_(lse[:, r0:r1, None]).exp_()
+        o[:, r0:r1] = p @ v
+        if do is not None:
+            g_o = do[:, r0:r1]
+            ds = (g_o @ v.T).sub_((g_o * o[:, r0:r1]).sum(-1, keepdim=True)).mul_(p).mul_(scale)
+            dq[:, r0:r1] = ds @ k
+            dk += (ds.transpose(1, 2) @ q[:, r0:r1]).sum(0)
+            dv += (p.transpose(1, 2) @ g_o).sum(0)
+    out = (o.transpose(0, 1), lse.T)
+    return out + (dq.transpose(0, 1), dk, dv) if do is not None else out
+
+
+def _visible(c, n, b, h):
+    """Mask of the rows [r0, r1) of sequence b, head h, over its n keys."""
+    j = torch.arange(n, device="cuda")
+    if c["kind"] == "blocks":
+        lists = c["idx"][b, h].long()
+        nb = lists.shape[0]
+        blocks = torch.zeros(nb, nb + 1, dtype=torch.bool, device="cuda")     # the last column takes the padding
+        blocks.scatter_(1, torch.where(lists < 0, nb, lists), True)
+
+    def mask(r0, r1):
+        i = torch.arange(r0, r1, device="cuda")[:, None]
+        if c["kind"] == "prefill" and not c["causal"]:
+            return torch.ones(1, r1 - r0, n, dtype=torch.bool, device="cuda")
+        m = j <= i
+        if c["kind"] == "window":
+            m = m & ((i - j < c["local"]) | (j < c["glob"]))
+        elif c["kind"] == "blocks":
+            m = m & blocks[i // BLOCK, j // BLOCK]
+        return m[None]
+    return mask
+
+
+def exact(case, seed):
+    """What `run(prepare(case, seed))` returns, computed by plain torch in 64 bits."""
+    s = prepare(case, seed)
+    c = s["case"]
+    kind = c["kind"]
+    if kind == "rmsnorm":
+        x, w = (s[n].detach().double() for n in "xw")
+        dy = s["dy"].double()
+        r = (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+        gw = dy * w
+        return x * r * w, r * (gw - x * r * r * (gw * x).mean(-1, keepdim=True)), (dy * x * r).sum(0)
+    g, scale = c["hq"] // c["hkv"], c["d"] ** -0.5
+    if kind in ("prefill", "blocks", "packed", "train", "window"):
+        q, k, v = (s[n].detach() for n in "qkv")
+        do = s.get("do")
+        if kind == "prefill":
+            spans = [(b, 0, c["seq"]) for b in range(c["batch"])]
+        else:
+            at = s["cu"].tolist()
+            spans = [(0, at[b], at[b + 1]) for b in range(c["batch"])]
+        o, lse = q.new_empty(q.shape, dtype=torch.float64), q.new_empty(q.shape[:3], dtype=torch.float64)
+        grads = [t.new_empty(t.shape, dtype=torch.float64) for t in (q, k, v)] if do is not None else []
+        each = 1 if kind == "blocks" else g     # a block list belongs to one query head
+        for b, (row, lo, hi) in enumerate(spans):
+            for h in range(0, c["hq"], each):
+                hs, hk = slice(h, h + each), h // g
+                mask = _visible(dict(c, idx=s.get("idx")), hi - lo, b, h)
+                r = _attend(q[row, lo:hi, hs], k[row, lo:hi, hk], v[row, lo:hi, hk], mask, scale,
+                            do[row, lo:hi, hs] if do is not None else None)
+                o[row, lo:hi, hs], lse[row, lo:hi, hs] = r[:2]
+                if do is not None:
+                    grads[0][row, lo:hi, hs], grads[1][row, lo:hi, hk], grads[2][row, lo:hi, hk] = r[2:]
+        if kind == "train":
+            return (o, *grads)
+        return o, lse / math.log(2) if kind == "window" else lse
+    k, v = s["k"], s["v"]
+    if kind == "decode_step":
+        lens = [n + 1 for n in _lens(c)]
+        for b, n in enumerate(lens):
+            k[b, n - 1], v[b, n - 1] = s["new_k"][b], s["new_v"][b]
+    elif kind == "topk":
+        lens = [c["seq"]] * c["batch"]
+        scores = s["scores"].clone()
+        scores[..., -1] = math.inf
+        idx = scores.topk(c["top_k"], -1).indices.sort(-1).values
+    else:
+        lens = _lens(c)
+    o = s["q"].new_empty(s["q"].shape, dtype=torch.float64)
+    for b, n in enumerate(lens):
+        if kind == "paged":
+            at = s["table"][b, :-(-n // c["page"])].long()
+            kb, vb = (t[at].flatten(0, 1)[:n] for t in (k, v))
+        else:
+            kb, vb = k[b, :n], v[b, :n]
+        j = torch.arange(n, device="cuda")
+        m = torch.ones(1, 1, n, dtype=torch.bool, device="cuda")
+        if kind == "window_decode":
+            m = ((j < c["glob"]) | (j >= n - c["local"]))[None, None]
+        for h in range(c["hkv"]):
+            if kind == "topk":
+                listed_ = torch.zeros(n // BLOCK, dtype=torch.bool, device="cuda")
+                listed_[idx[b, h]] = True
+                m = listed_[j // BLOCK][None, None]
+            o[b, h * g:(h + 1) * g] = _attend(s["q"][b:b + 1, h * g:(h + 1) * g], kb[:, h], vb[:, h],
+                                              lambda r0, r1: m, scale)[0][0]
+    if kind == "decode_step":
+        return o, k.double(), v.double()
+    if kind == "topk":
+        return o, idx.int(), torch.full(idx.shape[:2], c["top_k"], dtype=torch.int32, device="cuda")
+    return o
