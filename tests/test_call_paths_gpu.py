@@ -1,0 +1,95 @@
+"""The native call path against the Python one it stands before."""
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    from tritonops_b200 import ops
+    return ops
+
+
+def _packed(lens, hq, hkv, d, dtype, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    q, k, v, do = (torch.randn(1, sum(lens), h, d, generator=g, device="cuda").to(dtype) for h in (hq, hkv, hkv, hq))
+    return q, k, v, do, cu
+
+
+def test_native_calls_equal_python_calls(monkeypatch):
+    """Same bits from both paths over the argument forms the native one takes, and the forms it
+    leaves to Python (strided, other integer types, lengths on the CPU) still work."""
+    ops = _ops()
+    q, k, v, do, cu = _packed([70, 200, 33], 8, 2, 128, torch.bfloat16)
+    wide = torch.cat([q, q], 3)[..., :128]                       # strided rows
+    odd = torch.cat([q.new_zeros(1, q.shape[1], 8, 1), q], 3)[..., 1:]   # rows that are not 16-byte addressable
+    kc, vc = (torch.randn(3, 300, 2, 128, device="cuda").bfloat16() for _ in range(2))
+    qd, lens = q[0, :3].contiguous(), torch.tensor([300, 5, 64], dtype=torch.int32, device="cuda")
+    table = torch.arange(15, device="cuda", dtype=torch.int32).view(3, 5).flip(1).contiguous()
+    x, w = torch.randn(40, 512, device="cuda"), torch.rand(512, device="cuda")
+    scores = torch.randn(2, 3, 40, device="cuda")
+
+    def results():
+        out = []
+        for qq in (q, wide, odd):
+            for c in (cu, cu.long(), cu.cpu()):
+                out += ops.prefill(qq, k, v, cu_seqlens=c)
+        o, lse = ops.prefill(q, k, v, cu_seqlens=cu, window_local=50, window_global=3, sparsity=ops.WINDOW)
+        out += [o, lse, *ops.prefill_bwd(q, k, v, *[out[0]], do, out[1], cu_seqlens=cu)[1:]]
+        out += ops.prefill(kc, kc, vc, causal=False, scale=0.2)
+        out += [ops.decode(qd, kc, vc, seqlens=lens), ops.decode(qd, kc, vc, cu_seqlens=cu[:4].contiguous())]
+        out.append(ops.paged_decode(qd, kc[:, :256].reshape(12, 64, 2, 128)[:12].repeat(2, 1, 1, 1)[:15],
+                                    vc[:, :256].reshape(12, 64, 2, 128)[:12].repeat(2, 1, 1, 1)[:15], table, lens))
+        k2, v2 = kc.clone(), vc.clone()
+        ops.append_kv(k2, v2, k[0, :3].contiguous(), v[0, :3].contiguous(), lens)
+        out += [k2, v2, *ops.topk_blocks(scores, 7, force_last=1), *ops.topk_blocks(scores[0, 0], 7)]
+        for xx in (x, x.view(4, 10, 512), x[::2], x.bfloat16()):
+            y, r = ops.rmsnorm_fwd(xx, w, 1e-6)
+            out += [y, r, *ops.rmsnorm_bwd(y, xx, w, r)]
+        return out
+
+    native = results()
+    n = ops.launch_counter
+    ops.prefill(q, k, v, cu_seqlens=cu)
+    assert ops.launch_counter == n + 1
+    monkeypatch.setattr(ops, "_native", lambda *a: None)
+    python = results()
+    assert len(native) == len(python)
+    for i, (a, b) in enumerate(zip(native, python)):
+        assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride() and torch.equal(a, b), i
+
+
+def test_native_calls_raise_what_python_calls_raise():
+    ops = _ops()
+    q, k, v, _, cu = _packed([64], 4, 4, 64, torch.float16)
+    for bad, exc in [((q, k[..., :32], v), ValueError), ((q.float(), k, v), ValueError), ((q.cpu(), k, v), RuntimeError),
+                     ((q, k[:, :, :3], v[:, :, :3]), ValueError)]:
+        with pytest.raises(exc):
+            ops.prefill(*bad, cu_seqlens=cu)
+    with pytest.raises(ValueError):
+        ops.prefill(q.repeat(2, 1, 1, 1), k, v, cu_seqlens=cu)
+
+
+def test_first_call_of_a_thread_with_cached_memory():
+    """A thread that has made no CUDA call yet, all of whose allocations come from the cache."""
+    ops = _ops()
+    q, k, v, do, cu = _packed([64], 2, 2, 64, torch.float16)
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu)
+    ops.prefill_bwd(q, k, v, o, do, lse, cu_seqlens=cu)
+    torch.cuda.synchronize()
+    for call in (lambda: ops.prefill(q, k, v, cu_seqlens=cu), lambda: ops.prefill_bwd(q, k, v, o, do, lse, cu_seqlens=cu),
+                 lambda: ops.decode(q[0, :1], k, v, seqlens=cu[1:].contiguous())):
+        failed = []
+
+        def run():
+            try:
+                call()
+            except Exception as e:      # noqa: BLE001 - whatever it is, the test reports it
+                failed.append(e)
+        t = threading.Thread(target=run)
+        t.start()
+        t.join()
+        assert not failed, failed

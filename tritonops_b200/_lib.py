@@ -3,10 +3,13 @@
 There is no fallback: if the shared library is missing or a call fails, the
 Python layer raises."""
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libb200attn.so")
+HOST_PATH = os.path.join(_HERE, "csrc", "_b200host.so")
 
 F16, BF16, F32 = 0, 1, 2
 DENSE, WINDOW, BLOCK_LIST = 0, 1, 2
@@ -153,6 +156,24 @@ SYMBOLS = {
 NOALLOC_SCRATCH_BYTES = 32 << 20
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native call path of ops.py (csrc/host.cpp), bound to the library; raises if it has not
+    been built."""
+    global _host
+    if _host is None:
+        path = LIB_PATH
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m tritonops_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_b200host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200host", loader))
+        loader.exec_module(module)
+        module.init(path)
+        _host = module
+    return _host
 
 
 def lib():

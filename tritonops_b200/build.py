@@ -1,13 +1,16 @@
-"""Build libb200attn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Build libb200attn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and the native
+call path of the tensor-level entry points (_b200host.so, against the installed torch).
 
     python -m tritonops_b200.build [--force]
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 LIB = os.path.join(CSRC, "libb200attn.so")
+HOST = os.path.join(CSRC, "_b200host.so")
 SOURCES = ["api.cu", "decode.cu", "prefill.cu", "prefill_bwd.cu", "kvcache.cu", "blocksel.cu", "rmsnorm.cu", "selftest.cu"]
 HEADERS = ["common.cuh", os.path.join("..", "..", "include", "b200attn.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -15,11 +18,11 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 
 
 def _stale():
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(HOST):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
     deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS]
-    deps += [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".cu"))]
+    deps += [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".cu", ".cpp"))]
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
@@ -34,7 +37,23 @@ def build_library(force=False, verbose=False):
         sys.stderr.write(res.stderr)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+    build_host()
     return LIB
+
+
+def build_host():
+    """Compile csrc/host.cpp into csrc/_b200host.so."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           f"-I{sysconfig.get_paths()['include']}", "-o", HOST, "host.cpp",
+           f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{root}/lib"]
+    res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("host build failed:\n" + res.stdout + res.stderr)
 
 
 if __name__ == "__main__":

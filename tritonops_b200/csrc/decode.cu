@@ -795,15 +795,16 @@ template <typename T, int DP>
 static int launch_decode_tma_d(const b200attn_decode_args* a, const DecodeParams& p, dim3 g1, dim3 g2,
                                cudaStream_t stream) {
   using L = DecodeTmaSmem<DP>;
+  auto kern = decode_split_tma_kernel<T, DP>;
+  // per device and cheap, so set on every call rather than remembered (and before the
+  // tensor maps: it makes the device's context current on this thread, which their encoder needs)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
   CUtensorMap tk, tv;
   if (!make_cache_tmap(&tk, a->dtype, a->k_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch,
                        a->k_stride_t, a->k_stride_h, a->k_stride_b) ||
       !make_cache_tmap(&tv, a->dtype, a->v_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch,
                        a->v_stride_t, a->v_stride_h, a->v_stride_b))
-    return B200ATTN_ERR_CUDA;
-  auto kern = decode_split_tma_kernel<T, DP>;
-  // per device and cheap, so set on every call rather than remembered
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
     return B200ATTN_ERR_CUDA;
   kern<<<g1, 160, L::kAlloc, stream>>>(tk, tv, p);
   cudaError_t e;

@@ -835,12 +835,6 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
   using L = PrefillSmem<DP, BN, NSTAGE>;
   const long long tokens = a->cu_seqlens ? a->total_tokens : a->seqlen;
   const int tb = a->cu_seqlens ? 1 : a->batch;
-  CUtensorMap tq, tk, tv, to;
-  if (!make_tmap(&tq, a->dtype, a->q, a->head_dim, tokens, a->heads_q, tb, a->q_stride_t, a->q_stride_h, a->q_stride_b, kTileM) ||
-      !make_tmap(&tk, a->dtype, a->k, a->head_dim, tokens, a->heads_kv, tb, a->k_stride_t, a->k_stride_h, a->k_stride_b, p.block_idx ? kBlk : BN) ||
-      !make_tmap(&tv, a->dtype, a->v, a->head_dim, tokens, a->heads_kv, tb, a->v_stride_t, a->v_stride_h, a->v_stride_b, p.block_idx ? kBlk : BN) ||
-      !make_tmap(&to, a->dtype, a->o, a->head_dim, tokens, a->heads_q, tb, a->o_stride_t, a->o_stride_h, a->o_stride_b, kTileM))
-    return B200ATTN_ERR_CUDA;
   auto kern = p.block_idx ? prefill_kernel<T, DP, BN, NSTAGE, true> : prefill_kernel<T, DP, BN, NSTAGE, false>;
   // the register count is a property of the binary: checked once per instantiation and mode
   static std::once_flag regs_once[2];
@@ -853,8 +847,16 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
                             : B200ATTN_ERR_CUDA;   // fewer registers: the hand-over would not balance
   });
   if (regs_status[mode] != B200ATTN_OK) return regs_status[mode];
-  // the shared-memory opt-in is per device: set on every call (a process may drive several GPUs)
+  // the shared-memory opt-in is per device: set on every call (a process may drive several GPUs).
+  // Before the tensor maps: it makes the device's context current on this thread, which their encoder
+  // needs -- an autograd thread whose allocations all came from a cache may have made no CUDA call yet.
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
+  CUtensorMap tq, tk, tv, to;
+  if (!make_tmap(&tq, a->dtype, a->q, a->head_dim, tokens, a->heads_q, tb, a->q_stride_t, a->q_stride_h, a->q_stride_b, kTileM) ||
+      !make_tmap(&tk, a->dtype, a->k, a->head_dim, tokens, a->heads_kv, tb, a->k_stride_t, a->k_stride_h, a->k_stride_b, p.block_idx ? kBlk : BN) ||
+      !make_tmap(&tv, a->dtype, a->v, a->head_dim, tokens, a->heads_kv, tb, a->v_stride_t, a->v_stride_h, a->v_stride_b, p.block_idx ? kBlk : BN) ||
+      !make_tmap(&to, a->dtype, a->o, a->head_dim, tokens, a->heads_q, tb, a->o_stride_t, a->o_stride_h, a->o_stride_b, kTileM))
     return B200ATTN_ERR_CUDA;
   const long long blocks = (long long)p.pair_count * a->heads_q * a->batch;
   if (blocks <= 0) return B200ATTN_OK;

@@ -713,6 +713,11 @@ int launch_bwd(const b200attn_prefill_bwd_args* a, const BwdParams& p, cudaStrea
   using L = BwdSmem<DP>;
   const long long tokens = a->cu_seqlens ? a->total_tokens : a->seqlen;
   const int tb = a->cu_seqlens ? 1 : a->batch;
+  // (first: it makes the device's context current on this thread, which the tensor-map encoder needs --
+  // an autograd thread whose allocations all came from a cache may have made no CUDA call yet)
+  auto kern = bwd_kernel<T, DP>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
   CUtensorMap tq, tk, tv, tdo, tdk, tdv;
   if (!make_tmap(&tq, a->dtype, a->q, a->head_dim, tokens, a->heads_q, tb, a->q_stride_t, a->q_stride_h, a->q_stride_b) ||
       !make_tmap(&tk, a->dtype, a->k, a->head_dim, tokens, a->heads_kv, tb, a->k_stride_t, a->k_stride_h, a->k_stride_b) ||
@@ -720,9 +725,6 @@ int launch_bwd(const b200attn_prefill_bwd_args* a, const BwdParams& p, cudaStrea
       !make_tmap(&tdo, a->dtype, a->d_o, a->head_dim, tokens, a->heads_q, tb, a->do_stride_t, a->do_stride_h, a->do_stride_b) ||
       !make_tmap(&tdk, a->dtype, a->dk, a->head_dim, tokens, a->heads_kv, tb, a->dk_stride_t, a->dk_stride_h, a->dk_stride_b) ||
       !make_tmap(&tdv, a->dtype, a->dv, a->head_dim, tokens, a->heads_kv, tb, a->dv_stride_t, a->dv_stride_h, a->dv_stride_b))
-    return B200ATTN_ERR_CUDA;
-  auto kern = bwd_kernel<T, DP>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
     return B200ATTN_ERR_CUDA;
   const long long rows = total_rows(a);
   CUtensorMap tdq;

@@ -80,6 +80,21 @@ def _count():
     launch_counter += _lib.lib().b200attn_last_launch_count()
 
 
+def _native(name: str, *args):
+    """The call in native code (csrc/host.cpp): its outputs, or None where that path leaves the
+    call to the Python one below it (unusual tensors, a compiler or the debug mode at work)."""
+    global launch_counter
+    if DEBUG_STATUS or torch.compiler.is_compiling():
+        return None
+    r = getattr(_lib.host(), name)(*args)
+    if r is None:
+        return None
+    if type(r) is int:
+        _lib.check(r)
+    launch_counter += r[0]
+    return r[1:]
+
+
 def _stream(t: Tensor):
     return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
@@ -176,11 +191,15 @@ def decode(q, k_cache, v_cache, *, cu_seqlens=None, seqlens=None, max_seqlen=Non
     """Split-KV GQA decoding; see b200attn_decode_fwd in include/b200attn.h."""
     if (cu_seqlens is None) == (seqlens is None):
         raise ValueError("give exactly one of cu_seqlens and seqlens")
-    lens = _i32(cu_seqlens if cu_seqlens is not None else seqlens, q.device)
     if scale is None:
         scale = q.shape[-1] ** -0.5
     if max_seqlen is None:
         max_seqlen = k_cache.shape[1]
+    r = _native("decode", q, k_cache, v_cache, seqlens if cu_seqlens is None else cu_seqlens, cu_seqlens is not None,
+                max_seqlen, scale, chunk, sparsity, window_global, window_local, block_idx, block_cnt, block_size)
+    if r is not None:
+        return r[0]
+    lens = _i32(cu_seqlens if cu_seqlens is not None else seqlens, q.device)
     fn = _decode_op if torch.compiler.is_compiling() else _decode_op_impl   # eager: skip the dispatcher
     return fn(q, k_cache, v_cache, lens, cu_seqlens is not None, int(max_seqlen),
                       float(scale), int(chunk), int(sparsity), int(window_global),
@@ -192,6 +211,9 @@ def paged_decode(q: Tensor, k_pages: Tensor, v_pages: Tensor, page_table: Tensor
                  max_seqlen: Optional[int] = None, scale: Optional[float] = None, chunk: int = 0) -> Tensor:
     """Split-KV GQA decoding over page pools [num_pages, page_size, Hkv, D] addressed through
     page_table int32 [B, max_pages]; see b200attn_paged_decode_fwd in include/b200attn.h."""
+    r = _native("paged_decode", q, k_pages, v_pages, page_table, seqlens, max_seqlen, scale, chunk)
+    if r is not None:
+        return r[0]
     _same_head_dim(q, k_pages, v_pages)
     _need_cuda(q, k_pages, v_pages, page_table, seqlens)
     if q.dtype not in _DT or k_pages.dtype != q.dtype or v_pages.dtype != q.dtype:
@@ -272,6 +294,9 @@ def topk_blocks(scores: Tensor, top_k: int, *, n_valid: Optional[Tensor] = None,
                 force_last: int = 0) -> Tuple[Tensor, Tensor]:
     """Per row of fp32 `scores` [..., n_blocks]: the top_k best candidate blocks in ascending block
     order, (block_idx [..., top_k] padded with -1, block_cnt [...])."""
+    r = _native("topk_blocks", scores, top_k, n_valid, force_first, force_last)
+    if r is not None:
+        return r
     _need_cuda(scores, n_valid)
     if scores.dtype != torch.float32:
         raise ValueError("b200attn: block scores must be float32")
@@ -388,22 +413,32 @@ def _(q, k, v, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal, lse_base2
             q.new_empty(q.shape[:3], dtype=torch.float32))
 
 
+def _longest(cu: Tensor) -> int:
+    """Length of the longest sequence: the one host sync of the reference wrapper
+    (flash_attn_triton.py:621); pass max_seqlen to avoid it."""
+    return int((cu[1:] - cu[:-1]).max().item()) if cu.numel() > 1 else 0
+
+
 def prefill(q, k, v, *, cu_seqlens=None, max_seqlen=None, scale=None, scale_has_log2e=False,
             causal=True, lse_base2=False, sparsity=DENSE, window_local=0, window_global=0,
             block_idx=None, block_cnt=None, block_size=64) -> Tuple[Tensor, Tensor]:
     """Prefill attention forward -> (o, lse); see b200attn_prefill_fwd in include/b200attn.h.
 
     q [Bt, T, Hq, D]; with cu_seqlens the tensors are packed ([1, total, H, D])."""
-    cu = _i32(cu_seqlens, q.device)
     if scale is None:
         scale, scale_has_log2e = q.shape[-1] ** -0.5, False
+    if max_seqlen is None and cu_seqlens is None:
+        max_seqlen = q.shape[1]
+    if max_seqlen is None and cu_seqlens.is_cuda and cu_seqlens.dtype == torch.int32:
+        max_seqlen = _longest(cu_seqlens)
+    if max_seqlen is not None:
+        r = _native("prefill", q, k, v, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal, lse_base2, sparsity,
+                    window_local, window_global, block_idx, block_cnt, block_size)
+        if r is not None:
+            return r
+    cu = _i32(cu_seqlens, q.device)
     if max_seqlen is None:
-        if cu is not None:
-            # the one host sync of the reference wrapper (flash_attn_triton.py:621);
-            # pass max_seqlen to avoid it
-            max_seqlen = int((cu[1:] - cu[:-1]).max().item()) if cu.numel() > 1 else 0
-        else:
-            max_seqlen = q.shape[1]
+        max_seqlen = _longest(cu)
     fn = _prefill_op if torch.compiler.is_compiling() else _prefill_op_impl   # eager: skip the dispatcher
     return fn(q, k, v, cu, int(max_seqlen), float(scale), bool(scale_has_log2e),
                        bool(causal), bool(lse_base2), int(sparsity), int(window_local),
@@ -470,14 +505,20 @@ def prefill_bwd(q, k, v, o, d_o, lse, *, cu_seqlens=None, max_seqlen=None, scale
                 scale_has_log2e=False, causal=True, lse_base2=False):
     """Gradients (dq, dk, dv) of the dense prefill; see b200attn_prefill_bwd in include/b200attn.h.
     `o`, `lse` are the forward's outputs (lse in the form given by `lse_base2`)."""
-    cu = _i32(cu_seqlens, q.device)
     if scale is None:
         scale, scale_has_log2e = q.shape[-1] ** -0.5, False
+    if max_seqlen is None and cu_seqlens is None:
+        max_seqlen = q.shape[1]
+    if max_seqlen is None and cu_seqlens.is_cuda and cu_seqlens.dtype == torch.int32:
+        max_seqlen = _longest(cu_seqlens)
+    if max_seqlen is not None:
+        r = _native("prefill_bwd", q, k, v, o, d_o, lse, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal,
+                    lse_base2)
+        if r is not None:
+            return r
+    cu = _i32(cu_seqlens, q.device)
     if max_seqlen is None:
-        if cu is not None:
-            max_seqlen = int((cu[1:] - cu[:-1]).max().item()) if cu.numel() > 1 else 0
-        else:
-            max_seqlen = q.shape[1]
+        max_seqlen = _longest(cu)
     fn = _prefill_bwd_op if torch.compiler.is_compiling() else _prefill_bwd_op_impl
     return fn(q, k, v, o, d_o, lse, cu, int(max_seqlen), float(scale),
                            bool(scale_has_log2e), bool(causal), bool(lse_base2))
@@ -514,6 +555,8 @@ def pack_kv_cache(packed: Tensor, cu_seqlens: Tensor, capacity: int, out: Option
 
 def append_kv(k_cache: Tensor, v_cache: Tensor, new_k: Tensor, new_v: Tensor, seqlens: Tensor) -> None:
     """In place: cache[b, seqlens[b]] = new[b] for K and V (one decoding step)."""
+    if _native("append_kv", k_cache, v_cache, new_k, new_v, seqlens) is not None:
+        return
     _need_cuda(k_cache, v_cache, new_k, new_v, seqlens)
     if k_cache.stride() != v_cache.stride() or new_k.stride() != new_v.stride():
         raise ValueError("b200attn: K and V caches (and new rows) must share their strides")
@@ -549,6 +592,9 @@ def _rms_dtypes(x: Tensor, weight: Tensor):
 
 def rmsnorm_fwd(x: Tensor, weight: Tensor, eps: float) -> Tuple[Tensor, Tensor]:
     """(y like x, rstd fp32 [rows]); see b200attn_rmsnorm_fwd in include/b200attn.h."""
+    r = _native("rmsnorm_fwd", x, weight, eps)
+    if r is not None:
+        return r
     _need_cuda(x, weight)
     xd, wd = _rms_dtypes(x, weight)
     x2, w = _rows_view(x), weight.contiguous()
@@ -568,6 +614,9 @@ def rmsnorm_fwd(x: Tensor, weight: Tensor, eps: float) -> Tuple[Tensor, Tensor]:
 
 def rmsnorm_bwd(dy: Tensor, x: Tensor, weight: Tensor, rstd: Tensor) -> Tuple[Tensor, Tensor]:
     """(dx like x, dweight like weight); see b200attn_rmsnorm_bwd in include/b200attn.h."""
+    r = _native("rmsnorm_bwd", dy, x, weight, rstd)
+    if r is not None:
+        return r
     _need_cuda(dy, x, weight, rstd)
     xd, wd = _rms_dtypes(x, weight)
     if dy.dtype != x.dtype:
