@@ -1,4 +1,5 @@
-"""The native call path against the Python one it stands before."""
+"""The native call path against the Python one it stands before, and the device-side schedule of
+packed launches against single-sequence calls."""
 import threading
 
 import pytest
@@ -17,6 +18,50 @@ def _packed(lens, hq, hkv, d, dtype, seed=0):
     cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
     q, k, v, do = (torch.randn(1, sum(lens), h, d, generator=g, device="cuda").to(dtype) for h in (hq, hkv, hkv, hq))
     return q, k, v, do, cu
+
+
+# ragged batches on both sides of the schedule's limits: one lane per sequence (32), several chunks
+# of sequences, more sequences than are handed out on the device (256), heads that do not fill a
+# group of 8, tiles of exactly one, just under and just over 128 / 256 rows, empty sequences
+@pytest.mark.parametrize("lens,hq,hkv,d", [
+    ([256, 1, 0, 255, 257, 700, 128], 12, 12, 128),
+    ([(37 * i) % 300 for i in range(45)], 4, 2, 64),
+    ([1 + (91 * i) % 140 for i in range(260)], 2, 1, 64),
+    ([3000, 17], 9, 3, 96),
+])
+def test_packed_schedule_equals_single_sequences(lens, hq, hkv, d):
+    """Every tile of every sequence is computed exactly once: bit-equal to calls that hold one
+    sequence each (a tile's arithmetic does not depend on which CTA runs it)."""
+    ops = _ops()
+    q, k, v, do, cu = _packed(lens, hq, hkv, d, torch.bfloat16)
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu)
+    om, lsem = ops.prefill(q, k, v, cu_seqlens=cu, max_seqlen=max(lens))
+    assert torch.equal(o, om) and torch.equal(lse, lsem)
+    dq, dk, dv = ops.prefill_bwd(q, k, v, o, do, lse, cu_seqlens=cu)
+    at = cu.tolist()
+    for b, n in enumerate(lens):
+        if n == 0 or (len(lens) > 60 and b % 37):
+            continue
+        s = slice(at[b], at[b + 1])
+        one = [t[:, s].contiguous() for t in (q, k, v, do)]
+        o1, l1 = ops.prefill(*one[:3])
+        assert torch.equal(o[:, s], o1) and torch.equal(lse[:, s], l1), (b, n)
+        dq1, dk1, dv1 = ops.prefill_bwd(*one[:3], o1, one[3], l1)
+        assert torch.equal(dk[:, s], dk1) and torch.equal(dv[:, s], dv1), (b, n)
+        # dq is summed by reduce-adds in arrival order: one rounding of the 16-bit result
+        assert (dq[:, s].float() - dq1.float()).abs().max() <= 2 ** -7 * dq1.float().abs().max()
+
+
+def test_packed_call_without_lengths_can_be_captured():
+    """No length goes back to the host any more: the call fits into a CUDA graph."""
+    ops = _ops()
+    q, k, v, _, cu = _packed([100, 300], 4, 2, 128, torch.float16)
+    want = ops.prefill(q, k, v, cu_seqlens=cu)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.prefill(q, k, v, cu_seqlens=cu)
+    graph.replay()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
 def test_native_calls_equal_python_calls(monkeypatch):

@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "schedule.cuh"
 #include "sm100.cuh"
 
 namespace b200attn {
@@ -60,6 +61,7 @@ struct PrefillParams {
   int batch, heads_q, heads_kv, group, head_dim;
   int seqlen, n_pairs;
   int pair_begin, pair_count;   // the 256-row query blocks this launch computes: [pair_begin, pair_begin + pair_count)
+  PackedGrid packed;    // packed.seqs > 0: CTAs are handed out by packed_item
   int prefetch_ahead;   // CTAs resident at once: a CTA asks for the first tiles of CTA + this into L2
   int causal, window, win_local, win_global;
   float scale_log2;
@@ -216,14 +218,26 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   // kHeadGroup: inside a group the heaviest query blocks of all its heads come
   // first (longest-first keeps the tail of the launch short), and the group is
   // small enough that its K/V stay in L2 while its CTAs are resident.
+  // Packed launches get theirs from packed_item (the same order over the tiles that exist).
   const int n_bh = p.batch * p.heads_q;
   const int per_group = kHeadGroup * p.pair_count;
-  const int grp = blockIdx.x / per_group;
-  const int in_grp = blockIdx.x - grp * per_group;
-  const int g_heads = min(kHeadGroup, n_bh - grp * kHeadGroup);
-  const int pair = p.pair_begin + p.pair_count - 1 - in_grp / g_heads;
-  const int bh = grp * kHeadGroup + in_grp % g_heads;
-  const int h = bh % p.heads_q, b = bh / p.heads_q;
+  auto locate = [&](int bid, int& b_, int& h_, int& pair_) -> bool {
+    if (p.packed.seqs > 0) {
+      PackedItem it;
+      if (!packed_item(p.packed, p.cu_seqlens, p.batch, kPairM, p.n_pairs, p.heads_q, bid, it)) return false;
+      b_ = it.b; h_ = it.head; pair_ = it.level;
+      return true;
+    }
+    const int grp = bid / per_group;
+    const int in_grp = bid - grp * per_group;
+    const int g_heads = min(kHeadGroup, n_bh - grp * kHeadGroup);
+    pair_ = p.pair_begin + p.pair_count - 1 - in_grp / g_heads;
+    const int bh = grp * kHeadGroup + in_grp % g_heads;
+    h_ = bh % p.heads_q; b_ = bh / p.heads_q;
+    return true;
+  };
+  int b, h, pair;
+  if (!locate(blockIdx.x, b, h, pair)) return;
   const int hk = h / p.group;
   int seq_start = 0, len = p.seqlen, bcoord = b;
   if (p.cu_seqlens) {
@@ -371,13 +385,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // spends ~2.5 us before its first product can start.  Issued behind this CTA's own
       // first loads (in front of them it delayed them: 1041 instead of 1086 TFLOP/s).
       auto prefetch_next_cta = [&]() {
-        if (p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x && elect_one()) {
-          const int bi = blockIdx.x + p.prefetch_ahead;
-          const int grp2 = bi / per_group, in2 = bi - grp2 * per_group;
-          const int gh2 = min(kHeadGroup, n_bh - grp2 * kHeadGroup);
-          const int pair2 = p.pair_begin + p.pair_count - 1 - in2 / gh2;
-          const int bh2 = grp2 * kHeadGroup + in2 % gh2;
-          const int h2 = bh2 % p.heads_q, b2 = bh2 / p.heads_q;
+        int b2, h2, pair2;
+        if (p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x &&
+            locate(blockIdx.x + p.prefetch_ahead, b2, h2, pair2) && elect_one()) {
           int ss2 = 0, len2 = p.seqlen, bc2 = b2;
           if (p.cu_seqlens) { ss2 = p.cu_seqlens[b2]; len2 = min(p.cu_seqlens[b2 + 1] - ss2, p.n_pairs * kPairM); bc2 = 0; }
           const int q02 = pair2 * kPairM;
@@ -858,7 +868,8 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
       !make_tmap(&tv, a->dtype, a->v, a->head_dim, tokens, a->heads_kv, tb, a->v_stride_t, a->v_stride_h, a->v_stride_b, p.block_idx ? kBlk : BN) ||
       !make_tmap(&to, a->dtype, a->o, a->head_dim, tokens, a->heads_q, tb, a->o_stride_t, a->o_stride_h, a->o_stride_b, kTileM))
     return B200ATTN_ERR_CUDA;
-  const long long blocks = (long long)p.pair_count * a->heads_q * a->batch;
+  const long long blocks = a->heads_q * (p.packed.seqs > 0 ? packed_tiles_bound(a->batch, a->total_tokens, kPairM, p.n_pairs)
+                                                           : (long long)p.pair_count * a->batch);
   if (blocks <= 0) return B200ATTN_OK;
   if (blocks > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
   kern<<<(unsigned)blocks, kPrefillThreads, L::kAlloc, stream>>>(tq, tk, tv, to, p);
@@ -885,6 +896,9 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
   p.n_pairs = (maxlen + kPairM - 1) / kPairM;
   // a row range ends on a 256-row boundary unless it runs to the end of the longest sequence
   if (!all_rows && row_end < maxlen && row_end % kPairM != 0) return B200ATTN_ERR_SHAPE;
+  p.packed = PackedGrid{0, 0};
+  if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch)
+    p.packed = packed_grid(a->batch, a->total_tokens, (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
   p.pair_begin = row_begin / kPairM;
   p.pair_count = (int)std::min<long long>(p.n_pairs, ((long long)row_end + kPairM - 1) / kPairM) - p.pair_begin;
   if (p.pair_count <= 0) return B200ATTN_OK;

@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "schedule.cuh"
 #include "sm100.cuh"
 
 namespace b200attn {
@@ -55,6 +56,7 @@ struct BwdParams {
   int causal;
   float scale_log2, scale;   // q.k multiplier in base-2 and natural form
   int lse_base2;
+  PackedGrid packed;         // packed.seqs > 0: CTAs are handed out by packed_item
   int prefetch_ahead;        // CTAs resident at once: a CTA asks for the first tiles of CTA + this into L2
   int* status_word;
 };
@@ -68,17 +70,23 @@ struct BwdParams {
 #endif
 constexpr int kBwdHeadGroup = B200ATTN_BWD_HEAD_GROUP;
 struct BwdCta { int jt, hk, b; };
-__device__ __forceinline__ BwdCta bwd_cta_of(const BwdParams& p, int bid) {
+// (executed by whole converged warps; false: a packed launch has fewer tiles than CTAs)
+__device__ __forceinline__ bool bwd_cta_of(const BwdParams& p, int bid, BwdCta& c) {
+  if (p.packed.seqs > 0) {
+    PackedItem it;
+    if (!packed_item(p.packed, p.cu_seqlens, p.batch, kT, p.n_kvtiles, p.heads_kv, bid, it)) return false;
+    c.b = it.b; c.hk = it.head; c.jt = it.n_tiles - 1 - it.level;
+    return true;
+  }
   const int n_bh = p.batch * p.heads_kv;
   const int per_group = kBwdHeadGroup * p.n_kvtiles;
   const int grp = bid / per_group, in_grp = bid - grp * per_group;
   const int g_heads = min(kBwdHeadGroup, n_bh - grp * kBwdHeadGroup);
   const int bh = grp * kBwdHeadGroup + in_grp % g_heads;
-  BwdCta c;
   c.jt = in_grp / g_heads;
   c.hk = bh % p.heads_kv;
   c.b = bh / p.heads_kv;
-  return c;
+  return true;
 }
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -122,7 +130,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
   constexpr uint32_t kIdDQ = idesc_f16(kFmt, true, kT, DP, true);      // dQ: A, B MN-major
   constexpr int kPanels = DP / 64;
 
-  const BwdCta me = bwd_cta_of(p, blockIdx.x);
+  BwdCta me;
+  if (!bwd_cta_of(p, blockIdx.x, me)) return;
   const int jt = me.jt;                      // key tile
   const int hk = me.hk, b = me.b;
   int seq_start = 0, len = p.seqlen, bcoord = b;
@@ -186,6 +195,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
   auto pair_of = [&](int it, int& i, int& hq) { i = i_first + it / p.group; hq = hk * p.group + it % p.group; };
   if (warp == kBwdLoadWarp) {
     // ============================================ loader warp: every load, and the dQ reduce-adds
+    BwdCta nx;     // the CTA that will start when one of the resident ones ends
+    const bool have_nx = p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x &&
+                         bwd_cta_of(p, blockIdx.x + p.prefetch_ahead, nx);
     if (elect_one()) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_do);
       int n_q[2] = {0, 0}, n_do[2] = {0, 0};     // loads sent into each buffer so far
@@ -216,10 +228,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
         tma_load_4d(sbase + L::kV + pn * L::kPanel, &tmap_v, bar_kv, 64 * pn, seq_start + kv0, hk, bcoord);
       load_do(0);
       if (n_iter > 1) { load_q(1); load_do(1); }
-      // The CTA that will start when one of the resident ones ends finds its K / V tile and its
-      // first Q / dO tiles on their way into L2.
-      if (p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x) {
-        const BwdCta nx = bwd_cta_of(p, blockIdx.x + p.prefetch_ahead);
+      // That next CTA finds its K / V tile and its first Q / dO tiles on their way into L2.
+      if (have_nx) {
         int ss2 = 0, len2 = p.seqlen, bc2 = nx.b;
         if (p.cu_seqlens) { ss2 = p.cu_seqlens[nx.b]; len2 = min(p.cu_seqlens[nx.b + 1] - ss2, p.n_kvtiles * kT); bc2 = 0; }
         if (nx.jt * kT < len2) {
@@ -739,7 +749,8 @@ int launch_bwd(const b200attn_prefill_bwd_args* a, const BwdParams& p, cudaStrea
         a->heads_q, a->head_dim, DP, rows);
   }
   // 2. main kernel (the dq accumulator was cleared by the row-sum kernel)
-  const long long n_ctas = (long long)p.n_kvtiles * a->heads_kv * a->batch;
+  const long long n_ctas = a->heads_kv * (p.packed.seqs > 0 ? packed_tiles_bound(a->batch, a->total_tokens, kT, p.n_kvtiles)
+                                                            : (long long)p.n_kvtiles * a->batch);
   if (n_ctas > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
   dim3 grid((unsigned)n_ctas);
   kern<<<grid, kBwdThreads, L::kAlloc, stream>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
@@ -789,6 +800,10 @@ int prefill_bwd(const b200attn_prefill_bwd_args* a, cudaStream_t stream) {
   const int maxlen = a->cu_seqlens ? a->max_seqlen : a->seqlen;
   p.n_kvtiles = (maxlen + kT - 1) / kT;
   if (p.n_kvtiles <= 0) return B200ATTN_OK;
+  p.packed = PackedGrid{0, 0};
+  if (a->cu_seqlens && a->batch <= kSchedMaxBatch)
+    // what should stay in L2 here is the fp32 dQ accumulator of the head group (and its Q, dO)
+    p.packed = packed_grid(a->batch, a->total_tokens, (long long)kSchedHeads * p.group * dpad(a->head_dim) * 8);
   p.causal = a->causal ? 1 : 0;
   p.scale = a->softmax_scale * (a->scale_has_log2e ? 0.6931471805599453f : 1.f);
   p.scale_log2 = a->softmax_scale * (a->scale_has_log2e ? 1.f : 1.4426950408889634f);

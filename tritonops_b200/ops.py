@@ -413,6 +413,17 @@ def _(q, k, v, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal, lse_base2
             q.new_empty(q.shape[:3], dtype=torch.float32))
 
 
+# packed batches of at most this many sequences are handed out on the device from their lengths
+# (kSchedMaxBatch of csrc/schedule.cuh); the longest length then bounds nothing the launch needs
+_ANY_LENGTH_BATCH = 256
+
+
+def _any_length(cu_seqlens: Tensor, sparsity: int = DENSE) -> bool:
+    """May the total number of tokens stand in for the longest sequence's length?  (Block lists are
+    refused by length, so there the length has to be the true one.)"""
+    return cu_seqlens.numel() - 1 <= _ANY_LENGTH_BATCH and sparsity != BLOCK_LIST
+
+
 def _longest(cu: Tensor) -> int:
     """Length of the longest sequence: the one host sync of the reference wrapper
     (flash_attn_triton.py:621); pass max_seqlen to avoid it."""
@@ -427,10 +438,8 @@ def prefill(q, k, v, *, cu_seqlens=None, max_seqlen=None, scale=None, scale_has_
     q [Bt, T, Hq, D]; with cu_seqlens the tensors are packed ([1, total, H, D])."""
     if scale is None:
         scale, scale_has_log2e = q.shape[-1] ** -0.5, False
-    if max_seqlen is None and cu_seqlens is None:
+    if max_seqlen is None and (cu_seqlens is None or _any_length(cu_seqlens, sparsity)):
         max_seqlen = q.shape[1]
-    if max_seqlen is None and cu_seqlens.is_cuda and cu_seqlens.dtype == torch.int32:
-        max_seqlen = _longest(cu_seqlens)
     if max_seqlen is not None:
         r = _native("prefill", q, k, v, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal, lse_base2, sparsity,
                     window_local, window_global, block_idx, block_cnt, block_size)
@@ -507,10 +516,8 @@ def prefill_bwd(q, k, v, o, d_o, lse, *, cu_seqlens=None, max_seqlen=None, scale
     `o`, `lse` are the forward's outputs (lse in the form given by `lse_base2`)."""
     if scale is None:
         scale, scale_has_log2e = q.shape[-1] ** -0.5, False
-    if max_seqlen is None and cu_seqlens is None:
+    if max_seqlen is None and (cu_seqlens is None or _any_length(cu_seqlens)):
         max_seqlen = q.shape[1]
-    if max_seqlen is None and cu_seqlens.is_cuda and cu_seqlens.dtype == torch.int32:
-        max_seqlen = _longest(cu_seqlens)
     if max_seqlen is not None:
         r = _native("prefill_bwd", q, k, v, o, d_o, lse, cu_seqlens, max_seqlen, scale, scale_has_log2e, causal,
                     lse_base2)
