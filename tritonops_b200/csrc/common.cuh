@@ -45,6 +45,25 @@ int rmsnorm_fwd(const b200attn_rmsnorm_fwd_args* a, cudaStream_t stream);
 size_t rmsnorm_bwd_workspace_bytes(const b200attn_rmsnorm_bwd_args* a);
 int rmsnorm_bwd(const b200attn_rmsnorm_bwd_args* a, cudaStream_t stream);
 
+// Launch allowed to begin while the kernel before it on the stream drains; the kernel itself waits
+// (sm100::grid_dependency_wait) before it touches global memory.  Its set-up and the launch gap then
+// run under that kernel's tail: a one-CTA prefill replayed back to back takes 5.4 us instead of 6.4,
+// the four launches of a small training step (9 x 100-2500 tokens) 190 us instead of 198.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // 16-byte read-only load that does not pollute L1 (data is used once).
 template <typename T>
 __device__ __forceinline__ uint4 ld_nc_16(const T* ptr) {

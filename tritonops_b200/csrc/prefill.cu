@@ -227,6 +227,39 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   constexpr uint32_t kIdescPV = idesc_f16(kFmt, true, kTileM, DP);
   constexpr int kPanels = DP / 64;
 
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t sQ = smem_base;
+  const uint32_t sKV = smem_base + 2 * L::kQBytes;
+  const uint32_t bars = smem_base + L::kBarOffset;
+  auto q_full = [&](int t) { return bars + 8 * t; };
+  auto kv_full = [&](int s) { return bars + 8 * (2 + s); };
+  auto kv_empty = [&](int s) { return bars + 8 * (2 + NSTAGE + s); };
+  auto s_full = [&](int t) { return bars + 8 * (2 + 2 * NSTAGE + t); };
+  auto p_full = [&](int t) { return bars + 8 * (4 + 2 * NSTAGE + t); };
+  auto o_full = [&](int t) { return bars + 8 * (6 + 2 * NSTAGE + t); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kBarOffset + L::kNumBars * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kBarOffset + L::kNumBars * 8 + 4);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(q_full(t), 1);
+      mbar_init(s_full(t), 1);
+      mbar_init(p_full(t), 4);
+      mbar_init(o_full(t), 1);
+    }
+    for (int s = 0; s < NSTAGE; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  // (launched with programmatic stream serialisation: the set-up above runs while the kernel
+  // before this one drains, and the next one may begin when the last CTAs of this one have)
+  launch_dependents();
+  grid_dependency_wait();
+
   // ---- which 256 query rows.  (sequence, head) pairs are taken in groups of
   // kHeadGroup: inside a group the heaviest query blocks of all its heads come
   // first (longest-first keeps the tail of the launch short), and the group is
@@ -263,34 +296,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   if (q0 >= len) return;
   const TileSeq seq = make_seq<BN>(p, q0, len);
 
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t sQ = smem_base;
-  const uint32_t sKV = smem_base + 2 * L::kQBytes;
-  const uint32_t bars = smem_base + L::kBarOffset;
-  auto q_full = [&](int t) { return bars + 8 * t; };
-  auto kv_full = [&](int s) { return bars + 8 * (2 + s); };
-  auto kv_empty = [&](int s) { return bars + 8 * (2 + NSTAGE + s); };
-  auto s_full = [&](int t) { return bars + 8 * (2 + 2 * NSTAGE + t); };
-  auto p_full = [&](int t) { return bars + 8 * (4 + 2 * NSTAGE + t); };
-  auto o_full = [&](int t) { return bars + 8 * (6 + 2 * NSTAGE + t); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kBarOffset + L::kNumBars * 8);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kBarOffset + L::kNumBars * 8 + 4);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    *abort_flag = 0;
-    for (int t = 0; t < 2; ++t) {
-      mbar_init(q_full(t), 1);
-      mbar_init(s_full(t), 1);
-      mbar_init(p_full(t), 4);
-      mbar_init(o_full(t), 1);
-    }
-    for (int s = 0; s < NSTAGE; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
-    fence_barrier_init();
-    fence_proxy_async();
-  }
   if (warp == 0) {
     __syncwarp();
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
@@ -877,7 +882,8 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
                                                            : (long long)p.pair_count * a->batch);
   if (blocks <= 0) return B200ATTN_OK;
   if (blocks > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
-  kern<<<(unsigned)blocks, kPrefillThreads, L::kAlloc, stream>>>(tq, tk, tv, to, p);
+  if (launch_after(kern, dim3((unsigned)blocks), dim3(kPrefillThreads), L::kAlloc, stream, tq, tk, tv, to, p) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
   set_launch_count(1);
   return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
 }

@@ -130,23 +130,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
   constexpr uint32_t kIdDQ = idesc_f16(kFmt, true, kT, DP, true);      // dQ: A, B MN-major
   constexpr int kPanels = DP / 64;
 
-  BwdCta me;
-  if (!bwd_cta_of(p, blockIdx.x, me)) return;
-  const int jt = me.jt;                      // key tile
-  const int hk = me.hk, b = me.b;
-  int seq_start = 0, len = p.seqlen, bcoord = b;
-  if (p.cu_seqlens) {
-    seq_start = p.cu_seqlens[b];
-    // a sequence longer than the max_seqlen the grid was sized for is cut there
-    len = min(p.cu_seqlens[b + 1] - seq_start, p.n_kvtiles * kT);
-    bcoord = 0;
-  }
-  const int kv0 = jt * kT;
-  if (kv0 >= len) return;
-  const int n_qtiles = (len + kT - 1) / kT;
-  const int i_first = p.causal ? jt : 0;     // first query tile that sees this key tile
-  const int n_iter = (n_qtiles - i_first) * p.group;
-
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
@@ -177,6 +160,26 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
     fence_barrier_init();
     fence_proxy_async();
   }
+  launch_dependents();       // the conversion kernel may be set up; this one sees the row sums after the wait
+  grid_dependency_wait();
+
+  BwdCta me;
+  if (!bwd_cta_of(p, blockIdx.x, me)) return;
+  const int jt = me.jt;                      // key tile
+  const int hk = me.hk, b = me.b;
+  int seq_start = 0, len = p.seqlen, bcoord = b;
+  if (p.cu_seqlens) {
+    seq_start = p.cu_seqlens[b];
+    // a sequence longer than the max_seqlen the grid was sized for is cut there
+    len = min(p.cu_seqlens[b + 1] - seq_start, p.n_kvtiles * kT);
+    bcoord = 0;
+  }
+  const int kv0 = jt * kT;
+  if (kv0 >= len) return;
+  const int n_qtiles = (len + kT - 1) / kT;
+  const int i_first = p.causal ? jt : 0;     // first query tile that sees this key tile
+  const int n_iter = (n_qtiles - i_first) * p.group;
+
   if (warp == 0) {
     __syncwarp();
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
@@ -591,6 +594,8 @@ __global__ void bwd_rowsum_kernel(const T* __restrict__ o, const T* __restrict__
                                   float* __restrict__ dq_acc, long long o_sb, long long o_st, long long o_sh,
                                   long long do_sb, long long do_st, long long do_sh, int tokens_per_batch, int heads,
                                   int D, int DP, long long total) {
+  launch_dependents();
+  grid_dependency_wait();
   const int sub = threadIdx.x & 7;
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   float s = 0.f;
@@ -622,6 +627,7 @@ template <typename T>
 __global__ void bwd_convert_dq_kernel(const float* __restrict__ acc, T* __restrict__ dq, long long dq_sb,
                                       long long dq_st, long long dq_sh, int tokens_per_batch, int heads, int D,
                                       int DP, long long total_rows) {
+  grid_dependency_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // one thread per 8 elements
   const int per_row = DP / 8;
   const long long r = idx / per_row;
@@ -743,23 +749,26 @@ int launch_bwd(const b200attn_prefill_bwd_args* a, const BwdParams& p, cudaStrea
   // 1. D = rowsum(dO o O), and the dq accumulator cleared
   {
     const long long blocks = (rows * 8 + 255) / 256;
-    bwd_rowsum_kernel<T><<<(unsigned)blocks, 256, 0, stream>>>(
+    if (launch_after(bwd_rowsum_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, stream,
         (const T*)a->o, (const T*)a->d_o, const_cast<float*>(p.dvec), p.dq_acc, a->cu_seqlens ? 0 : a->o_stride_b,
         a->o_stride_t, a->o_stride_h, a->cu_seqlens ? 0 : a->do_stride_b, a->do_stride_t, a->do_stride_h, tpb,
-        a->heads_q, a->head_dim, DP, rows);
+        a->heads_q, a->head_dim, DP, rows) != cudaSuccess)
+      return B200ATTN_ERR_CUDA;
   }
   // 2. main kernel (the dq accumulator was cleared by the row-sum kernel)
   const long long n_ctas = a->heads_kv * (p.packed.seqs > 0 ? packed_tiles_bound(a->batch, a->total_tokens, kT, p.n_kvtiles)
                                                             : (long long)p.n_kvtiles * a->batch);
   if (n_ctas > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
   dim3 grid((unsigned)n_ctas);
-  kern<<<grid, kBwdThreads, L::kAlloc, stream>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  if (launch_after(kern, grid, dim3(kBwdThreads), L::kAlloc, stream, tq, tk, tv, tdo, tdq, tdk, tdv, p) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
   // 3. dq accumulator -> dq
   {
     const long long items = rows * (DP / 8);
-    bwd_convert_dq_kernel<T><<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(
+    if (launch_after(bwd_convert_dq_kernel<T>, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream,
         p.dq_acc, (T*)a->dq, a->cu_seqlens ? 0 : a->dq_stride_b, a->dq_stride_t, a->dq_stride_h, tpb,
-        a->heads_q, a->head_dim, DP, rows);
+        a->heads_q, a->head_dim, DP, rows) != cudaSuccess)
+      return B200ATTN_ERR_CUDA;
   }
   set_launch_count(3);
   return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
