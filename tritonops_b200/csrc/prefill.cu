@@ -205,7 +205,7 @@ struct PrefillSmem {
   static constexpr int kStageBytes = BN * DP * 2;
   static constexpr int kKvPanel = BN * 128;
   static constexpr int kBarOffset = 2 * kQBytes + NSTAGE * kStageBytes;
-  static constexpr int kNumBars = 2 + 2 * NSTAGE + 6;
+  static constexpr int kNumBars = 2 + 2 * NSTAGE + 8;
   // block-list mode: 4 bitmaps (one per 64-row query block of the CTA), then per
   // query tile the merged ascending list of KV blocks with a 2-bit membership mask
   static constexpr int kBitmapOffset = kBarOffset + kNumBars * 8 + 16;
@@ -226,6 +226,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   constexpr uint32_t kIdescQK = idesc_f16(kFmt, false, kTileM, BN);
   constexpr uint32_t kIdescPV = idesc_f16(kFmt, true, kTileM, DP);
   constexpr int kPanels = DP / 64;
+  // Narrow heads leave 128 columns of tensor memory over, which hold P beside S instead of over it:
+  // Q K^T of the next step is then issued as soon as the softmax warps have S in registers, and its
+  // time drops out of the chain S -> softmax -> P V (B=4 H=32 S=4096: 438 -> 429 us; block lists,
+  // B=2 H=16 S=8192: 186 -> 171 us).  With 128-wide heads S, S, O, O fill the 512 columns; one S shared
+  // by both tiles would make room there, and measured 2-3 % slower (514 against 499 us).
+  constexpr bool kAhead = DP == 64;
+  // Exponentials on the FMA pipe: one value in four for dense tiles of 128-wide heads (one in eight
+  // measured 1 % slower there), one in eight where the pass is short of issue slots rather than of
+  // MUFU (64-wide heads: 429 -> 423 us at B=4 H=32 S=4096; block lists, which skip the exponentials of
+  // unlisted halves: 620 -> 610 us at B=2 H=16 S=16384 D=128).
+  constexpr int kPolyMask = (!BLK && DP == 128) ? 2 : 6;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -239,6 +250,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   auto s_full = [&](int t) { return bars + 8 * (2 + 2 * NSTAGE + t); };
   auto p_full = [&](int t) { return bars + 8 * (4 + 2 * NSTAGE + t); };
   auto o_full = [&](int t) { return bars + 8 * (6 + 2 * NSTAGE + t); };
+  auto s_free = [&](int t) { return bars + 8 * (8 + 2 * NSTAGE + t); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kBarOffset + L::kNumBars * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kBarOffset + L::kNumBars * 8 + 4);
 
@@ -250,6 +262,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       mbar_init(s_full(t), 1);
       mbar_init(p_full(t), 4);
       mbar_init(o_full(t), 1);
+      mbar_init(s_free(t), 4);
     }
     for (int s = 0; s < NSTAGE; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
     fence_barrier_init();
@@ -306,7 +319,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   auto tS = [&](int t) { return tmem + 128u * t; };
-  auto tO = [&](int t) { return tmem + 256u + 128u * t; };
+  auto tO = [&](int t) { return tmem + 256u + (uint32_t)(DP * t); };
+  auto tP = [&](int t) { return kAhead ? tmem + 384u + 64u * t : tmem + 128u * t; };
 
   // ---- block-list mode: each 128-row query tile walks the union of the lists
   // of its two 64-row query blocks, two KV blocks per 128-key step, with its own
@@ -446,16 +460,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         // the first product needs Q of tile 0 and the first K tile: those two first, then Q of tile 1
         if (n_steps > 0) load_stage(&tmap_k, seq_start + seq.kv(0) * BN, 0, false);
         load_q(1);
-        for (int j = 0; j < n_steps; ++j) {
+        for (int j = 0; j < n_steps; ++j) {     // K of a step one V earlier when its product is issued ahead
           const int row = seq_start + seq.kv(j) * BN;
-          if (j > 0) load_stage(&tmap_k, row, 0, false);
+          if (kAhead && j + 1 < n_steps) load_stage(&tmap_k, seq_start + seq.kv(j + 1) * BN, 0, false);
+          if (!kAhead && j > 0) load_stage(&tmap_k, row, 0, false);
           load_stage(&tmap_v, row, 0, false);
           if (j == 1 || n_steps == 1) prefetch_next_cta();   // behind this CTA's own first loads
         }
       } else {
         load_q(1);
         // per tile its own stream, in the order the MMA warp consumes the stages:
-        // K(0,0) K(1,0), then per step V(0,j) K(0,j+1) V(1,j) K(1,j+1).  An odd
+        // K(0,0) K(1,0), then per step V(0,j) K(0,j+1) V(1,j) K(1,j+1), or each K before its V
+        // when the score product is issued ahead.  An odd
         // list repeats its last block in the second box (those columns are masked).
         auto load_blk = [&](const CUtensorMap* m, int t, int j) {
           const int nu = n_u[t];
@@ -466,10 +482,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         if (ns1 > 0) load_blk(&tmap_k, 1, 0);
         for (int j = 0; j < n_steps; ++j) {
           if (j == 1 || (j == 0 && n_steps == 1)) prefetch_next_cta();
-          if (j < ns0) load_blk(&tmap_v, 0, j);
-          if (j + 1 < ns0) load_blk(&tmap_k, 0, j + 1);
-          if (j < ns1) load_blk(&tmap_v, 1, j);
-          if (j + 1 < ns1) load_blk(&tmap_k, 1, j + 1);
+          for (int t = 0; t < 2; ++t) {
+            const int ns = t ? ns1 : ns0;
+            if (kAhead && j + 1 < ns) load_blk(&tmap_k, t, j + 1);
+            if (j < ns) load_blk(&tmap_v, t, j);
+            if (!kAhead && j + 1 < ns) load_blk(&tmap_k, t, j + 1);
+          }
         }
       }
       // every issued copy must have landed before the CTA may exit
@@ -484,7 +502,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     {
       const uint32_t issue = elect_one() ? 1u : 0u;
       int cnt = 0;
-      int pv_cnt[2] = {0, 0};
+      int pv_cnt[2] = {0, 0}, qk_cnt[2] = {0, 0};
       bool q_ready[2] = {false, false};
       // descriptors of stage 0 / tile 0; other stages and k-steps add to the address field
       const uint64_t dq0 = smem_desc_sw128(sQ, 16, 1024);
@@ -499,6 +517,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       };
       auto issue_qk = [&](int t, int s) {
         if (!q_ready[t]) { mbar_wait(q_full(t), 0, abort_flag); tc_fence_after(); q_ready[t] = true; }
+        if (kAhead) {     // the previous scores must be in registers
+          if (qk_cnt[t] > 0) { mbar_wait(s_free(t), (qk_cnt[t] - 1) & 1, abort_flag); tc_fence_after(); }
+          ++qk_cnt[t];
+        }
         const uint64_t da = dq0 + (uint64_t)((t * L::kQBytes) >> 4);
         const uint64_t db = dk0 + (uint64_t)((s * L::kStageBytes) >> 4);
         static_assert(BN == 128, "the grouped issue assumes 16 KB panels");
@@ -512,7 +534,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         mbar_wait(p_full(t), pv_cnt[t] & 1, abort_flag);
         tc_fence_after();
         const uint64_t db = dv0 + (uint64_t)((s * L::kStageBytes) >> 4);
-        mma_ts_x8(tO(t), tS(t), (uint32_t)db, (uint32_t)(db >> 32), kIdescPV, pv_cnt[t] > 0 ? 1u : 0u, issue);
+        mma_ts_x8(tO(t), tP(t), (uint32_t)db, (uint32_t)(db >> 32), kIdescPV, pv_cnt[t] > 0 ? 1u : 0u, issue);
         mma_commit(o_full(t), issue);
         ++pv_cnt[t];
       };
@@ -523,6 +545,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           if (n_steps > 0 && step_active(t, 0)) issue_qk(t, sK);
         if (n_steps > 0) mma_commit(kv_empty(sK), issue);
         for (int j = 0; j < n_steps; ++j) {
+          const bool more = j + 1 < n_steps;
+          int sKn = 0;
+          if (kAhead && more) {
+            sKn = wait_stage();
+            if (step_active(0, j + 1)) issue_qk(0, sKn);
+          }
           const int sV = wait_stage();
           // Rows of the V tile past the sequence end belong to the next packed sequence (or to
           // nobody): P is 0 there, but 0 * Inf/NaN would still poison O, so they are cleared
@@ -530,12 +558,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           if (seq.kv(j) * BN + BN > len)
             zero_tile_rows(smem_gen + 2 * L::kQBytes + sV * L::kStageBytes, kPanels, L::kKvPanel,
                            max(len - seq.kv(j) * BN, 0), BN, lane);
-          const bool more = j + 1 < n_steps;
-          int sKn = 0;
           for (int t = 0; t < 2; ++t) {
+            if (kAhead && t == 1 && more) {
+              if (step_active(1, j + 1)) issue_qk(1, sKn);
+              mma_commit(kv_empty(sKn), issue);
+            }
             if (step_active(t, j)) issue_pv(t, sV);
             if (t == 1) mma_commit(kv_empty(sV), issue);
-            if (more) {
+            if (!kAhead && more) {
               if (t == 0) sKn = wait_stage();
               if (step_active(t, j + 1)) issue_qk(t, sKn);
               if (t == 1) mma_commit(kv_empty(sKn), issue);
@@ -549,6 +579,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         for (int j = 0; j < n_steps; ++j) {
           for (int t = 0; t < 2; ++t) {
             const int ns = t ? ns1 : ns0;
+            if (kAhead && j + 1 < ns) { const int s = wait_stage(); issue_qk(t, s); mma_commit(kv_empty(s), issue); }
             if (j < ns) {
               const int s = wait_stage();
               // (rows past the sequence end inside the last KV block are cleared, see above)
@@ -561,7 +592,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
               issue_pv(t, s);
               mma_commit(kv_empty(s), issue);
             }
-            if (j + 1 < ns) { const int s = wait_stage(); issue_qk(t, s); mma_commit(kv_empty(s), issue); }
+            if (!kAhead && j + 1 < ns) { const int s = wait_stage(); issue_qk(t, s); mma_commit(kv_empty(s), issue); }
           }
         }
       }
@@ -589,6 +620,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 #pragma unroll
         for (int cc = 0; cc < BN / 32; ++cc) tmem_ld32(tS(t) + lane_off + 32 * cc, &sr[32 * cc]);
         tmem_wait_ld();
+        if (kAhead) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_free(t));
+        }
         bool vis0 = true, vis1 = true;   // does this warp's query block see each 64-column half?
         if (blk) {
           // columns [0,64) belong to KV block u0, [64,128) to u1; a row sees a
@@ -649,10 +685,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                           (m_run == -INFINITY && m_new != -INFINITY);
         const float m_use = grow ? m_new : m_run;
         const float alpha = (m_use == m_run) ? 1.f : ex2((m_run - m_use) * c);
-        if (items > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-          // O_t must hold every product issued so far before it is rescaled
+        const bool rescale = items > 0 && __any_sync(0xffffffffu, alpha != 1.f);
+        auto products_done = [&]() {      // O_t holds every product issued so far (and P has been read)
           mbar_wait(o_full(t), (items - 1) & 1, abort_flag);
           tc_fence_after();
+        };
+        auto rescale_o = [&]() {
 #pragma unroll
           for (int cc = 0; cc < DP / 32; ++cc) {
             uint32_t orr[32];
@@ -662,7 +700,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             for (int x = 0; x < 32; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
             tmem_st32(tO(t) + lane_off + 32 * cc, orr);
           }
-        }
+        };
+        if (!kAhead && rescale) { products_done(); rescale_o(); }
         const float mc = (m_use == -INFINITY) ? 0.f : m_use * c;
         float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
         uint32_t pr[BN / 2];
@@ -675,10 +714,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
               float e0, e1, e2, e3;
               ffma2(e0, e1, __uint_as_float(sr[2 * x]), __uint_as_float(sr[2 * x + 1]), c, neg_mc);
               ffma2(e2, e3, __uint_as_float(sr[2 * x + 2]), __uint_as_float(sr[2 * x + 3]), c, neg_mc);
-#ifndef B200ATTN_POLY_MASK
-#define B200ATTN_POLY_MASK 2
-#endif
-              if ((x & B200ATTN_POLY_MASK) == 0) {   // one value in four on the FMA pipe (more measured slower)
+              if ((x & kPolyMask) == 0) {
                 exp2_fma_pair(e0, e1, e0, e1);
               } else {
                 e0 = ex2(e0); e1 = ex2(e1);
@@ -693,10 +729,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 #pragma unroll
             for (int x = hb * (BN / 4); x < (hb + 1) * (BN / 4); ++x) pr[x] = 0u;
           }
+          if (kAhead) {
+            if (hb == 0 && items > 0) { products_done(); if (rescale) rescale_o(); }
+            tmem_st32(tP(t) + lane_off + 32 * hb, &pr[32 * hb]);
+          }
         }
         sum0 += sum2; sum1 += sum3;
+        if (!kAhead) {
 #pragma unroll
-        for (int cc = 0; cc < BN / 64; ++cc) tmem_st32(tS(t) + lane_off + 32 * cc, &pr[32 * cc]);
+          for (int cc = 0; cc < BN / 64; ++cc) tmem_st32(tP(t) + lane_off + 32 * cc, &pr[32 * cc]);
+        }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
