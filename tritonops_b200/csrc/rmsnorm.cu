@@ -198,6 +198,8 @@ rmsnorm_fwd_stream_kernel(const XT* __restrict__ x, const WT* __restrict__ w, XT
     fence_barrier_init();
     fence_proxy_async();
   }
+  launch_dependents();
+  grid_dependency_wait();     // (launched with programmatic stream serialisation)
   __syncthreads();
   auto slot_of = [&](long long it) { return (int)(it % n_slots); };
   auto use_of = [&](long long it) { return (uint32_t)((it / n_slots) & 1); };      // phase parity of row `it` in its slot
@@ -318,6 +320,8 @@ rmsnorm_bwd_stream_kernel(const XT* __restrict__ dy, const XT* __restrict__ x, c
     fence_barrier_init();
     fence_proxy_async();
   }
+  launch_dependents();
+  grid_dependency_wait();     // (launched with programmatic stream serialisation)
   __syncthreads();
   auto slot_of = [&](long long it) { return (int)(it % n_slots); };
   auto use_of = [&](long long it) { return (uint32_t)((it / n_slots) & 1); };      // phase parity of row `it` in its slot
@@ -592,13 +596,36 @@ rmsnorm_bwd_vec_kernel(const XT* __restrict__ dy, const XT* __restrict__ x, cons
   }
 }
 
+// dw[c] = sum of the partial rows' column c, in a fixed order: 32 columns per CTA, a warp per 32nd
+// partial row, so that a thread has a handful of independent loads instead of a chain of all rows
+// (148 partial rows of 4096 columns: 14 us with one thread per column).
+constexpr int kDwRows = 32;
 template <typename WT>
-__global__ void rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, WT* __restrict__ dw, int D, int n_partial) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D) return;
+__global__ void __launch_bounds__(32 * kDwRows)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, WT* __restrict__ dw, int D, int n_partial) {
+  sm100::grid_dependency_wait();
+  __shared__ float part[kDwRows][33];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int i = 0; i < n_partial; ++i) s += partial[(long long)i * D + c];
-  dw[c] = from_f<WT>(s);
+  if (c < D) {
+#pragma unroll 8
+    for (int i = r; i < n_partial; i += kDwRows) s += partial[(long long)i * D + c];
+  }
+  part[r][lane] = s;
+  __syncthreads();
+  // warp r adds the kDwRows sums of column r of this CTA
+  float t = part[lane][r];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  const int cr = blockIdx.x * 32 + r;
+  if (lane == 0 && cr < D) dw[cr] = from_f<WT>(t);
+}
+
+template <typename WT>
+cudaError_t launch_dw_reduce(const float* partial, void* dw, int D, int n_partial, cudaStream_t stream) {
+  return launch_after(rmsnorm_dw_reduce_kernel<WT>, dim3((D + 31) / 32), dim3(32 * kDwRows), 0, stream, partial,
+                      (WT*)dw, D, n_partial);
 }
 
 bool valid_dtypes(int xd, int wd) {
@@ -633,8 +660,10 @@ int launch_fwd(const b200attn_rmsnorm_fwd_args* a, cudaStream_t stream) {
     const int smem = StreamSmem::bytes(a->dim);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return B200ATTN_ERR_CUDA;
-    kern<<<grid, kFwdStreamThreads, smem, stream>>>((const XT*)a->x, (const WT*)a->weight, (XT*)a->y, a->rstd, a->rows,
-                                                  a->dim, a->x_stride_row, a->y_stride_row, a->eps, slot, n_slots);
+    if (launch_after(kern, dim3(grid), dim3(kFwdStreamThreads), smem, stream, (const XT*)a->x, (const WT*)a->weight,
+                     (XT*)a->y, a->rstd, a->rows, a->dim, a->x_stride_row, a->y_stride_row, a->eps, slot,
+                     n_slots) != cudaSuccess)
+      return B200ATTN_ERR_CUDA;
     set_launch_count(1);
     return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
   }
@@ -684,15 +713,17 @@ int launch_bwd_rms(const b200attn_rmsnorm_bwd_args* a, cudaStream_t stream) {
     auto kern = rmsnorm_bwd_stream_kernel<XT, WT, CH>;                                                            \
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)             \
       return B200ATTN_ERR_CUDA;                                                                                   \
-    kern<<<grid, kBwdStreamThreads, smem, stream>>>(dy, x, w, a->rstd, dx, partial, a->rows, a->dim, a->dy_stride_row, \
-                                                 a->x_stride_row, a->dx_stride_row, slot, n_slots);               \
+    if (launch_after(kern, dim3(grid), dim3(kBwdStreamThreads), smem, stream, dy, x, w, a->rstd, dx, partial,     \
+                     a->rows, a->dim, a->dy_stride_row, a->x_stride_row, a->dx_stride_row, slot,                  \
+                     n_slots) != cudaSuccess)                                                                     \
+      return B200ATTN_ERR_CUDA; \
   }
     if (ch <= 2) B200ATTN_RMS_BWD_STREAM(2)
     else if (ch <= 4) B200ATTN_RMS_BWD_STREAM(4)
     else if (ch <= 8) B200ATTN_RMS_BWD_STREAM(8)
     else if constexpr (N == 4) B200ATTN_RMS_BWD_STREAM(16)     // (fp32 rows: 4 columns per chunk)
 #undef B200ATTN_RMS_BWD_STREAM
-    rmsnorm_dw_reduce_kernel<WT><<<(a->dim + 255) / 256, 256, 0, stream>>>(partial, (WT*)a->dweight, a->dim, grid);
+    if (launch_dw_reduce<WT>(partial, a->dweight, a->dim, grid, stream) != cudaSuccess) return B200ATTN_ERR_CUDA;
     set_launch_count(2);
     return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
   }
@@ -711,7 +742,7 @@ int launch_bwd_rms(const b200attn_rmsnorm_bwd_args* a, cudaStream_t stream) {
   else
     rmsnorm_bwd_kernel<XT, WT, kBwdMaxCols><<<g, kBwdThreadsRms, 0, stream>>>(
         dy, x, w, a->rstd, dx, partial, a->rows, a->dim, a->dy_stride_row, a->x_stride_row, a->dx_stride_row);
-  rmsnorm_dw_reduce_kernel<WT><<<(a->dim + 255) / 256, 256, 0, stream>>>(partial, (WT*)a->dweight, a->dim, g);
+  if (launch_dw_reduce<WT>(partial, a->dweight, a->dim, g, stream) != cudaSuccess) return B200ATTN_ERR_CUDA;
   set_launch_count(2);
   return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
 }
