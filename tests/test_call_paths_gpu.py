@@ -1,5 +1,5 @@
-"""The native call path against the Python one it stands before, and the device-side schedule of
-packed launches against single-sequence calls."""
+"""The native call path against the Python one it stands before, the device-side schedule of packed
+launches against single-sequence calls, and one-chunk decoding against split decoding."""
 import threading
 
 import pytest
@@ -138,3 +138,26 @@ def test_first_call_of_a_thread_with_cached_memory():
         t.start()
         t.join()
         assert not failed, failed
+
+
+@pytest.mark.parametrize("d,dtype", [(128, torch.bfloat16), (64, torch.float16)])
+@pytest.mark.parametrize("lens", [[4096, 0, 1, 63, 64, 65, 4095], [130]])
+def test_one_chunk_decoding_equals_split_decoding(d, dtype, lens):
+    """max_seqlen within one chunk: the split kernel writes the output itself.  Against chunks of 64
+    keys: fp32 partial sums in another order, one rounding of the result (values below 4)."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    B, cap = len(lens), max(lens)
+    q = torch.randn(B, 8, d, generator=g, device="cuda").to(dtype)
+    k, v = (torch.randn(B, cap, 2, d, generator=g, device="cuda").to(dtype) for _ in range(2))
+    sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    one = ops.decode(q, k, v, seqlens=sl, chunk=4096)
+    many = ops.decode(q, k, v, seqlens=sl, chunk=64)
+    tol = 2 ** (-7 if dtype == torch.bfloat16 else -10) * 4
+    assert (one.float() - many.float()).abs().max() <= tol
+    if 0 in lens:
+        assert one[lens.index(0)].abs().max() == 0
+    # more items than fit the chip at once: the CTAs take over those that have not started
+    rep = 40
+    big = ops.decode(q.repeat(rep, 1, 1), k.repeat(rep, 1, 1, 1), v.repeat(rep, 1, 1, 1), seqlens=sl.repeat(rep), chunk=64)
+    assert torch.equal(big, many.repeat(rep, 1, 1))

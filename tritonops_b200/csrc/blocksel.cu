@@ -11,6 +11,7 @@
 // bound and exist so that no host round trip sits between the pattern's
 // producer and the attention launch.
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace b200attn {
 
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(kTopkThreads) topk_blocks_kernel(b200attn_topk
   __shared__ uint32_t s_prefix;
   __shared__ int s_remaining;
 
+  sm100::launch_dependents();   // a decoding kernel behind this one is set up meanwhile
   const int row = blockIdx.x;
   const int tid = threadIdx.x;
   int nv = a.n_valid ? a.n_valid[row] : a.n_blocks;
@@ -189,14 +191,30 @@ __global__ void __launch_bounds__(kTopkThreads) topk_blocks_kernel(b200attn_topk
         if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
       }
       __syncthreads();
-      if (tid == 0) {
-        int remaining = s_remaining, cum = 0, d = 255;
-        for (; d > 0; --d) {
-          if (cum + hist[d] >= remaining) break;
-          cum += hist[d];
+      // the largest digit with at least `remaining` keys at or above it: lane l of the first warp
+      // sums the eight digits from 255 - 8 l down, a scan finds the lane, which walks its eight
+      // (one thread walking the 256 counters took ~2 us a pass)
+      if (tid < 32) {
+        const int remaining = s_remaining;
+        int h[8], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { h[i] = hist[255 - 8 * tid - i]; sum += h[i]; }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (tid >= o) incl += t;
         }
-        s_remaining = remaining - cum;
-        s_prefix = prefix | ((uint32_t)d << shift);
+        int cum = incl - sum;
+        if (cum < remaining && incl >= remaining) {
+          int i = 0;
+          for (; i < 7; ++i) {
+            if (cum + h[i] >= remaining) break;
+            cum += h[i];
+          }
+          s_remaining = remaining - cum;
+          s_prefix = prefix | ((uint32_t)(255 - 8 * tid - i) << shift);
+        }
       }
       mask |= 255u << shift;
       __syncthreads();

@@ -23,6 +23,7 @@
 // 8 consecutive d of one token row (one 16-byte load) to the instruction:
 // the C fragment of S^T is, register for register, the B fragment of P^T.
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "sm100.cuh"
@@ -48,6 +49,8 @@ struct DecodeParams {
   long long q_sb, q_sh, k_sb, k_st, k_sh, v_sb, v_st, v_sh, o_sb, o_sh;
   int batch, heads_q, heads_kv, group, ggroups;
   int chunk, max_chunks;
+  int take_over;      // more CTAs than fit at once: a CTA takes over ones that have not started
+  int direct_o;       // one chunk per sequence: phase 1 writes o itself and there is no phase 2
   int sparsity, win_global, win_local, block_size, max_sel;
   int head_dim_rt;
   int max_seqlen;     // lengths beyond it are cut there (the grid and the scratch are sized for it)
@@ -72,7 +75,7 @@ struct KeyMap {
   __device__ __forceinline__ int to_token(int vpos) const {
     if (mode == 0) return vpos;
     if (mode == 1) return vpos < split ? vpos : vpos + shift;
-    int bi = vpos / bsize;
+    const int bi = bshift >= 0 ? vpos >> bshift : vpos / bsize;
     return blocks[bi] * bsize + (vpos - bi * bsize);
   }
 };
@@ -98,10 +101,12 @@ __device__ __forceinline__ KeyMap make_keymap(const DecodeParams& p, int b, int 
   } else if (p.sparsity == kPaged) {
     // key t lives in row page_table[b][t / page] * page + t % page of the pool
     m.bsize = p.block_size;
+    m.bshift = (m.bsize & (m.bsize - 1)) == 0 ? __ffs(m.bsize) - 1 : -1;
     m.blocks = p.block_idx + (long long)b * p.max_sel;
     m.n = min(m.len, p.max_sel * p.block_size);
   } else {
     m.bsize = p.block_size;
+    m.bshift = (m.bsize & (m.bsize - 1)) == 0 ? __ffs(m.bsize) - 1 : -1;
     m.blocks = p.block_idx + ((long long)b * p.heads_kv + hk) * p.max_sel;
     int cnt = p.block_cnt ? min(p.block_cnt[b * p.heads_kv + hk], p.max_sel) : p.max_sel;
     // trailing -1 entries are padding
@@ -328,17 +333,40 @@ decode_split_kernel(const DecodeParams p) {
 }
 
 // --------------------------------------------------------------------------
-// TMA variant of phase 1.  Same work split (one CTA per sequence, KV-head
-// group and 512-key chunk) and the same partials, but K and V reach the SM as
-// bulk tensor copies: a producer warp streams 64-key stages (four 16-key boxes
-// per operand and 64-column panel, 128-byte swizzle) through a shared-memory
-// ring guarded by full / empty mbarriers, so the bytes in flight per SM are set
-// by the ring depth rather than by the load/store unit's outstanding requests,
-// and four consumer warps read their 16 keys of each stage with ldmatrix.
-// Up to 16 query heads of a GQA group ride in one MMA tile (M = 16).
+// TMA variant of phase 1.  The work items are the same (sequence, KV-head group, chunk of keys)
+// and so are the partials, but K and V reach the SM as bulk tensor copies: a producer warp streams
+// 64-key stages (four 16-key boxes per operand and 64-column panel, 128-byte swizzle) through a
+// shared-memory ring guarded by full / empty mbarriers, so the bytes in flight per SM are set by
+// the ring depth rather than by the load/store unit's outstanding requests, and four consumer
+// warps read their 16 keys of each stage with ldmatrix.  Up to 16 query heads of a GQA group ride
+// in one MMA tile (M = 16).
+//
+// A CTA does not end with its item: it takes over CTAs of the launch that have not started yet
+// (cluster launch control) until none is left.  The producer asks for the next item while the
+// last stages of this one are on their way, and streams its first stages while the consumers are
+// still folding the previous chunk, so an item's set-up (length, block list, Q, first copies:
+// ~2 us in which a CTA per item moved no data) is hidden, and the hardware still hands out the
+// items one by one, which balances ragged batches.  Chunks are the slowest grid axis: those past
+// the end of short sequences come last.  A launch that fits the chip at once asks for nothing.
+// Where a stage's keys are consecutive rows one 64-key box per operand and panel brings them: 16
+// small boxes per stage were more than one thread could issue in the stage's time (a lone CTA:
+// 940 ns per stage, 690 ns with 4 boxes).
+// Measured, us of both phases before and after (bf16, D = 128, replayed from a graph): 24 sequences
+// of 300-6000 keys in pages of 64, 8 KV heads: 98 -> 60.5; 48 of 200-8000 in pages of 16: 174 -> 138;
+// 64 of 1024-8192, padded cache: 191 -> 185.5; top-64 blocks of 8 x 32 heads: 92 -> 84 (6.4 TB/s);
+// 100 of 200-2000, D = 64: 34 -> 26; one sequence of 3002 keys: 12.4 -> 9.7.
 // --------------------------------------------------------------------------
 constexpr int kStageTok = 64;   // keys per ring stage
 constexpr int kBoxTok = 16;     // keys per TMA box (window / block gathers are 16-key aligned)
+
+// one work item as the producer hands it to the consumers
+struct DecodeItem {
+  int x, b, chunk_id;     // grid coordinates: KV head and head group, sequence, chunk
+  int c_begin, c_end;     // its visible keys
+  int len;                // the sequence's length
+  int valid;              // 0: no more items
+  int pad;
+};
 
 template <int DP>
 struct DecodeTmaSmem {
@@ -347,11 +375,18 @@ struct DecodeTmaSmem {
   static constexpr int kTileBytes = kPanels * kPanelBytes;   // K or V of one stage
   static constexpr int kStageBytes = 2 * kTileBytes;
   static constexpr int kStages = DP == 128 ? 3 : 5;
-  static constexpr int kBarOffset = kStages * kStageBytes;
-  static constexpr int kBytes = kBarOffset + 2 * kStages * 8 + 16;
+  static constexpr int kQ = kStages * kStageBytes;           // the item's 16 query rows
+  static constexpr int kQPitch = DP * 2 + 16;                // bytes
+  static constexpr int kFold = kQ + 16 * kQPitch;            // [4 warps][16 heads][32 columns] or [8 heads][64], padded
+  static constexpr int kMl = kFold + 4 * 16 * 33 * 4;        // row max and sum, [2][4 warps][16 heads]
+  static constexpr int kTok = kMl + 2 * 4 * 16 * 4;          // cache row of each box of each stage
+  static constexpr int kItem = kTok + kStages * 16;
+  static constexpr int kNext = kItem + 32;                   // response of the launch control (16 bytes)
+  static constexpr int kBarOffset = kNext + 16;
+  static constexpr int kBytes = kBarOffset + (2 * kStages + 3) * 8 + 16;
   static constexpr int kAlloc = kBytes + 1024;
-  static constexpr int kCombinePitch = DP + 1;                // floats per (warp, head) row of the combine buffer
-  static_assert(4 * 16 * kCombinePitch * 4 + 2 * 4 * 16 * 4 <= kStages * kStageBytes, "combine buffer aliases the ring");
+  static_assert(kTok % 16 == 0 && kNext % 16 == 0 && kBarOffset % 8 == 0, "aligned");
+  static_assert(2 * (kAlloc + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3) {
@@ -363,283 +398,424 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, unsigned& r0, u
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
 
+// barrier of the 128 consumer threads; true if `flag` is for any of them
+__device__ __forceinline__ bool consumers_any(bool flag) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(flag ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
 template <typename T, int DP>
 __global__ void __launch_bounds__(160, 2)
 decode_split_tma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                        const __grid_constant__ CUtensorMap tmap_k64, const __grid_constant__ CUtensorMap tmap_v64,
                         const DecodeParams p) {
   using L = DecodeTmaSmem<DP>;
   using namespace sm100;
   constexpr int NKT = DP / 16;   // 16-wide d steps of the score product
   constexpr int NDT = DP / 8;    // 8-wide d tiles of the output
-  const int hk = blockIdx.x / p.ggroups;
-  const int gg = blockIdx.x % p.ggroups;   // group of 16 query heads inside the GQA group
-  const int chunk_id = blockIdx.y;
-  const int b = blockIdx.z;
-  const KeyMap km = make_keymap(p, b, hk);
-  const int c_begin = chunk_id * p.chunk;
-  if (c_begin >= km.n) return;
-  const int c_end = min(km.n, c_begin + p.chunk);
-  const int map_b = km.mode == kPaged ? 0 : b;   // a page pool has no batch axis
-  const int n_tiles = (c_end - c_begin + kStageTok - 1) / kStageTok;
-
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t bars = sbase + L::kBarOffset;
   auto full = [&](int s) { return bars + 8 * s; };
   auto empty = [&](int s) { return bars + 8 * (L::kStages + s); };
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kBarOffset + 2 * L::kStages * 8);
+  const uint32_t item_full = bars + 16 * L::kStages, item_empty = item_full + 8, next_full = item_full + 16;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kBarOffset + (2 * L::kStages + 3) * 8);
+  volatile DecodeItem* item = reinterpret_cast<volatile DecodeItem*>(sgen + L::kItem);
+  volatile int* box_tok = reinterpret_cast<volatile int*>(sgen + L::kTok);      // [stage][box]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Launched with programmatic stream serialisation: the set-up runs under the tail of the kernel
+  // before this one, and the combine kernel may be set up from here on (it waits for this grid).
+  launch_dependents();
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < L::kStages; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 4); }
+    mbar_init(item_full, 1);
+    mbar_init(item_empty, 4);
+    mbar_init(next_full, 1);
     fence_barrier_init();
     fence_proxy_async();
   }
+  if (threadIdx.x == 128) { prefetch_tmap(&tmap_k64); prefetch_tmap(&tmap_v64); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); }
+  grid_dependency_wait();
   __syncthreads();
 
+  // A wait by a whole warp, answered alike in all of its lanes (after a wait gave up somewhere, one
+  // lane might see its phase complete and another the abort flag).
+  auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool {
+    const bool done = mbar_wait(bar, parity, abort_flag);
+    return __all_sync(0xffffffffu, done);
+  };
   if (warp == 4) {
     // ================================================================ producer
-    if (lane == 0) {
-      prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      int issued = 0;
-      // Block lists and page tables: the block holding a stage's first key is looked up one
-      // stage ahead (the load is in flight during the wait for the stage to become free), and
-      // boxes of the stage that lie in the same block reuse it.
-      const bool listed = km.mode >= 2;
-      int nxt_blk = (listed && n_tiles > 0) ? km.blocks[c_begin / km.bsize] : 0;
-      for (int tile = 0; tile < n_tiles; ++tile, ++issued) {
-        const int s = tile % L::kStages;
+    int x = blockIdx.x, b = blockIdx.y, chunk_id = blockIdx.z;
+    int issued = 0;                       // stages sent so far, over all items
+    bool ok = true;
+    for (int n_item = 0; ok; ++n_item) {
+      bool asked = false;
+      const int hk = x / p.ggroups, gg = x - hk * p.ggroups;
+      const KeyMap km = make_keymap(p, b, hk);
+      const int c_begin = min(chunk_id * p.chunk, km.n);
+      const int c_end = min(km.n, c_begin + p.chunk);
+      const int n_tiles = (c_end - c_begin + kStageTok - 1) / kStageTok;
+      const int map_b = km.mode == kPaged ? 0 : b;   // a page pool has no batch axis
+      // the item's query rows into shared memory, and the item itself, once the consumers have
+      // taken the previous one's
+      constexpr int kVec = DP / 8;        // 16-byte pieces of a row
+      const T* qbase = (const T*)p.q + (long long)b * p.q_sb + (long long)(hk * p.group + gg * 16) * p.q_sh;
+      uint4 qv[16 * kVec / 32];
+#pragma unroll
+      for (int i = 0; i < 16 * kVec / 32; ++i) {
+        const int r = (lane + 32 * i) / kVec, c = (lane + 32 * i) % kVec;
+        qv[i] = (gg * 16 + r < p.group && 8 * c < p.head_dim_rt)
+                    ? *reinterpret_cast<const uint4*>(qbase + (long long)r * p.q_sh + 8 * c) : make_uint4(0, 0, 0, 0);
+      }
+      auto publish = [&]() -> bool {
+        if (!warp_wait(item_empty, (n_item & 1) ^ 1)) return false;
+#pragma unroll
+        for (int i = 0; i < 16 * kVec / 32; ++i) {
+          const int r = (lane + 32 * i) / kVec, c = (lane + 32 * i) % kVec;
+          *reinterpret_cast<uint4*>(sgen + L::kQ + r * L::kQPitch + 16 * c) = qv[i];
+        }
+        if (lane == 0) {
+          item->x = x; item->b = b; item->chunk_id = chunk_id;
+          item->c_begin = c_begin; item->c_end = c_end; item->len = km.len; item->valid = 1;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(item_full);
+        return true;
+      };
+      // The first item's copies leave before its query rows have arrived; later ones find the ring
+      // full of the item before.
+      const int publish_at = n_item == 0 ? min(n_tiles, L::kStages) - 1 : -1;
+      if (publish_at < 0) ok = publish();
+      // Lane i < 4 keeps the cache row of box i of the next stage: block lists and page tables are
+      // looked up a stage ahead, four boxes at once.
+      auto box_row = [&](int v) { return lane < kStageTok / kBoxTok && v < c_end ? km.to_token(v) : -1; };
+      int row_nx = box_row(c_begin + kBoxTok * lane);
+      for (int tile = 0; ok && tile < max(n_tiles, 1); ++tile) {
+        if (p.take_over && tile == max(n_tiles - 2, 0) && lane == 0) {   // what comes after this item
+          mbar_expect_tx(next_full, 16);
+          try_cancel_next_cta(sbase + L::kNext, next_full);
+          asked = true;
+        }
+        if (n_tiles == 0) break;
+        const int s = issued % L::kStages;
         const int v0 = c_begin + tile * kStageTok;
-        const int cur_blk = nxt_blk;
-        const int cur_idx = listed ? v0 / km.bsize : 0;
-        const int cur_off = listed ? v0 - cur_idx * km.bsize : 0;
-        if (listed && tile + 1 < n_tiles) nxt_blk = km.blocks[(v0 + kStageTok) / km.bsize];
-        if (!mbar_wait(empty(s), ((tile / L::kStages) & 1) ^ 1, abort_flag)) break;
-        const int nbox = min(kStageTok / kBoxTok, (c_end - v0 + kBoxTok - 1) / kBoxTok);
-        mbar_expect_tx(full(s), nbox * 2 * L::kPanels * kBoxTok * 128);
-        const uint32_t kdst = sbase + s * L::kStageBytes, vdst = kdst + L::kTileBytes;
-        for (int i = 0; i < nbox; ++i) {
-          // 16 consecutive cache rows (rows past the end are masked)
-          const int tok = (listed && cur_off + kBoxTok * i < km.bsize) ? cur_blk * km.bsize + cur_off + kBoxTok * i
-                                                                       : km.to_token(v0 + kBoxTok * i);
-          for (int pn = 0; pn < L::kPanels; ++pn) {
-            const uint32_t off = pn * L::kPanelBytes + i * kBoxTok * 128;
-            tma_load_4d(kdst + off, &tmap_k, full(s), 64 * pn, tok, hk, map_b);
-            tma_load_4d(vdst + off, &tmap_v, full(s), 64 * pn, tok, hk, map_b);
+        const int row = row_nx;
+        if (tile + 1 < n_tiles) row_nx = box_row(v0 + kStageTok + kBoxTok * lane);
+        int rows[kStageTok / kBoxTok];
+#pragma unroll
+        for (int i = 0; i < kStageTok / kBoxTok; ++i) rows[i] = __shfl_sync(0xffffffffu, row, i);
+        if (!warp_wait(empty(s), ((issued / L::kStages) & 1) ^ 1)) { ok = false; break; }
+        if (lane == 0) {
+          const uint32_t kdst = sbase + s * L::kStageBytes, vdst = kdst + L::kTileBytes;
+          const int nbox = min(kStageTok / kBoxTok, (c_end - v0 + kBoxTok - 1) / kBoxTok);
+#pragma unroll
+          for (int i = 0; i < kStageTok / kBoxTok; ++i) box_tok[4 * s + i] = rows[i];
+          mbar_expect_tx(full(s), nbox * 2 * L::kPanels * kBoxTok * 128);
+          if (nbox == 4 && rows[1] == rows[0] + 16 && rows[2] == rows[0] + 32 && rows[3] == rows[0] + 48) {
+            // 64 consecutive cache rows: one box per operand and panel
+            for (int pn = 0; pn < L::kPanels; ++pn) {
+              tma_load_4d(kdst + pn * L::kPanelBytes, &tmap_k64, full(s), 64 * pn, rows[0], hk, map_b);
+              tma_load_4d(vdst + pn * L::kPanelBytes, &tmap_v64, full(s), 64 * pn, rows[0], hk, map_b);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < kStageTok / kBoxTok; ++i) {
+              if (i >= nbox) break;
+              for (int pn = 0; pn < L::kPanels; ++pn) {     // 16 consecutive cache rows (rows past the end are masked)
+                const uint32_t off = pn * L::kPanelBytes + i * kBoxTok * 128;
+                tma_load_4d(kdst + off, &tmap_k, full(s), 64 * pn, rows[i], hk, map_b);
+                tma_load_4d(vdst + off, &tmap_v, full(s), 64 * pn, rows[i], hk, map_b);
+              }
+            }
           }
         }
+        __syncwarp();
+        ++issued;
+        if (tile == publish_at) ok = publish();
       }
-      // A wait gave up somewhere in the CTA: the consumers no longer wait for the stages, so
-      // the copies still in flight are waited for here before the CTA may exit.
-      if (*abort_flag)
-        for (int tile = max(issued - L::kStages, 0); tile < issued; ++tile)
-          mbar_drain(full(tile % L::kStages), (tile / L::kStages) & 1);
+      // (the answer writes shared memory, so it is waited for whatever happened)
+      asked = __shfl_sync(0xffffffffu, asked ? 1 : 0, 0) != 0;
+      if (!ok || (p.take_over && !warp_wait(next_full, n_item & 1))) {
+        if (asked) mbar_drain(next_full, n_item & 1);
+        break;
+      }
+      if (!p.take_over || !next_cta(sbase + L::kNext, x, b, chunk_id)) {
+        if (warp_wait(item_empty, n_item & 1)) {
+          if (lane == 0) { item->valid = 0; mbar_arrive(item_full); }
+        }
+        break;
+      }
+      __syncwarp();
+      fence_proxy_async();     // the answer has been read: the next request may overwrite it
     }
+    // A wait gave up somewhere in the CTA: the consumers no longer wait for the stages, so
+    // the copies still in flight are waited for here before the CTA may exit.
+    if (*abort_flag)
+      for (int i = max(issued - L::kStages, 0); i < issued; ++i) mbar_drain(full(i % L::kStages), (i / L::kStages) & 1);
     return;
   }
 
   // ================================================================== consumers
   const int gid = lane >> 2, tig = lane & 3;
-  const int g0 = gg * 16 + gid, g1 = g0 + 8;          // query heads of this lane's two MMA rows
-  const T* qbase = (const T*)p.q + (long long)b * p.q_sb + (long long)(hk * p.group) * p.q_sh;
-  unsigned qa[NKT][4];
+  const int D = p.head_dim_rt;
+  float* sm_fold = reinterpret_cast<float*>(sgen + L::kFold);
+  float* sm_m = reinterpret_cast<float*>(sgen + L::kMl);               // [4][16]
+  float* sm_l = sm_m + 4 * 16;
+  int used = 0;                            // stages read so far, over all items
+  for (int n_item = 0;; ++n_item) {
+    // (decided by all four warps together, here and below: a warp that left alone after a wait gave
+    // up would be missing from the others' barriers)
+    const bool got = mbar_wait(item_full, n_item & 1, abort_flag);
+    if (consumers_any(!got)) break;
+    if (!item->valid) break;
+    const int x = item->x, b = item->b, chunk_id = item->chunk_id;
+    const int c_begin = item->c_begin, c_end = item->c_end, len = item->len;
+    const int n_tiles = (c_end - c_begin + kStageTok - 1) / kStageTok;
+    const int hk = x / p.ggroups, gg = x - hk * p.ggroups;   // group of 16 query heads inside the GQA group
+    const int heads_here = min(16, p.group - gg * 16);
+    unsigned qa[NKT][4];                   // MMA rows gid and gid + 8
+    {
+      const uint32_t addr = sbase + L::kQ + ((lane & 7) + 8 * ((lane >> 3) & 1)) * L::kQPitch + 16 * (lane >> 4);
 #pragma unroll
-  for (int kt = 0; kt < NKT; ++kt) {
-    const int d = 16 * kt + 2 * tig;
-    const bool dok0 = d < p.head_dim_rt, dok1 = d + 8 < p.head_dim_rt;
-    qa[kt][0] = (g0 < p.group && dok0) ? *reinterpret_cast<const unsigned*>(qbase + (long long)g0 * p.q_sh + d) : 0u;
-    qa[kt][1] = (g1 < p.group && dok0) ? *reinterpret_cast<const unsigned*>(qbase + (long long)g1 * p.q_sh + d) : 0u;
-    qa[kt][2] = (g0 < p.group && dok1) ? *reinterpret_cast<const unsigned*>(qbase + (long long)g0 * p.q_sh + d + 8) : 0u;
-    qa[kt][3] = (g1 < p.group && dok1) ? *reinterpret_cast<const unsigned*>(qbase + (long long)g1 * p.q_sh + d + 8) : 0u;
-  }
-  float acc[NDT][4];
+      for (int kt = 0; kt < NKT; ++kt) ldmatrix_x4(addr + 32 * kt, qa[kt][0], qa[kt][1], qa[kt][2], qa[kt][3]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(item_empty);
+    if (n_tiles == 0) {                    // nothing visible in this chunk
+      if (p.max_chunks == 1 && p.direct_o) {
+        for (int idx = threadIdx.x; idx < heads_here * D; idx += 128) {
+          const int g = idx / D, d = idx - g * D;
+          ((T*)p.o)[(long long)b * p.o_sb + (long long)(hk * p.group + gg * 16 + g) * p.o_sh + d] = from_float<T>(0.f);
+        }
+      }
+      continue;
+    }
+    float acc[NDT][4];
 #pragma unroll
-  for (int i = 0; i < NDT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float l_run[2] = {0.f, 0.f};
+    for (int i = 0; i < NDT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    float m_run[2] = {-INFINITY, -INFINITY};
+    float l_run[2] = {0.f, 0.f};
 
-  for (int tile = 0; tile < n_tiles; ++tile) {
-    const int s = tile % L::kStages;
-    if (!mbar_wait(full(s), (tile / L::kStages) & 1, abort_flag)) break;   // reported below
-    const int v0 = c_begin + tile * kStageTok + 16 * warp;   // this warp's 16 keys of the stage
-    if (v0 < c_end) {
-      const uint32_t ktile = sbase + s * L::kStageBytes, vtile = ktile + L::kTileBytes;
-      // which of the 16 keys are real (inside the chunk and inside the sequence)
-      bool ok = false;
-      if (lane < 16) {
-        const int vp = v0 + lane;
-        if (vp < c_end) {
-          if (km.mode == kPaged) {
-            ok = true;                       // every key below the length is real, wherever its page lies
-          } else {
-            const int tok = km.to_token(v0 & ~(kBoxTok - 1)) + (lane & (kBoxTok - 1));
-            ok = tok >= 0 && tok < km.len;
+    for (int tile = 0; tile < n_tiles; ++tile, ++used) {
+      const int s = used % L::kStages;
+      if (!warp_wait(full(s), (used / L::kStages) & 1)) break;   // reported below
+      const int v0 = c_begin + tile * kStageTok + 16 * warp;   // this warp's 16 keys of the stage
+      if (v0 < c_end) {
+        const uint32_t ktile = sbase + s * L::kStageBytes, vtile = ktile + L::kTileBytes;
+        // which of the 16 keys are real (inside the chunk and inside the sequence; in a page pool
+        // every key below the length is real, wherever its page lies)
+        int n_real = min(c_end - v0, 16);
+        if (p.sparsity != kPaged) {
+          const int tok = box_tok[4 * s + warp];
+          n_real = tok >= 0 ? min(n_real, len - tok) : 0;
+        }
+        const unsigned vmask = n_real >= 16 ? 0xffffu : (n_real > 0 ? (1u << n_real) - 1u : 0u);
+        if (vmask != 0xffffu) {
+          // rows of V that are not real keys may hold anything (cache padding): P = 0
+          // times NaN would poison O, so they are cleared in shared memory first
+          uint8_t* vgen = sgen + (vtile - sbase);
+          for (int r = max(n_real, 0); r < 16; ++r) {
+            const int row = 16 * warp + r;
+            for (int i = lane; i < L::kPanels * 8; i += 32)
+              *reinterpret_cast<uint4*>(vgen + (i >> 3) * L::kPanelBytes + row * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async();   // these plain stores precede the copy engine's next write to the stage
+          __syncwarp();
+        }
+        // ---- S[g, key] = Q K^T for two 8-key tiles, even and odd d steps in sums of their own
+        // (a chain of NKT dependent MMAs is most of a stage's latency)
+        float ca[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        float cb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        {
+          const int mi = lane >> 3, r = lane & 7;
+          const int row = 16 * warp + 8 * (mi >> 1) + r;
+#pragma unroll
+          for (int kt = 0; kt < NKT; ++kt) {
+            const int c16 = 2 * kt + (mi & 1);
+            const uint32_t addr = ktile + (c16 >> 3) * L::kPanelBytes + row * 128 + (((c16 & 7) ^ (row & 7)) << 4);
+            unsigned b0, b1, b2, b3;
+            ldmatrix_x4(addr, b0, b1, b2, b3);
+            mma_16816<T>(ca[kt & 1], qa[kt][0], qa[kt][1], qa[kt][2], qa[kt][3], b0, b1);
+            mma_16816<T>(cb[kt & 1], qa[kt][0], qa[kt][1], qa[kt][2], qa[kt][3], b2, b3);
+          }
+        }
+        // columns of this thread: keys 2tig, 2tig+1 (ca) and 8+2tig, 9+2tig (cb); rows gid and gid+8
+        float sc[2][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          sc[r][0] = ((vmask >> (2 * tig)) & 1u) ? (ca[0][2 * r] + ca[1][2 * r]) * p.scale_log2 : -INFINITY;
+          sc[r][1] = ((vmask >> (2 * tig + 1)) & 1u) ? (ca[0][2 * r + 1] + ca[1][2 * r + 1]) * p.scale_log2 : -INFINITY;
+          sc[r][2] = ((vmask >> (8 + 2 * tig)) & 1u) ? (cb[0][2 * r] + cb[1][2 * r]) * p.scale_log2 : -INFINITY;
+          sc[r][3] = ((vmask >> (9 + 2 * tig)) & 1u) ? (cb[0][2 * r + 1] + cb[1][2 * r + 1]) * p.scale_log2 : -INFINITY;
+        }
+        float alpha[2];
+        unsigned pa[4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          float mx = fmaxf(fmaxf(sc[r][0], sc[r][1]), fmaxf(sc[r][2], sc[r][3]));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          const float m_new = fmaxf(m_run[r], mx);
+          const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+          alpha[r] = exp2f(m_run[r] - m_use);
+          m_run[r] = m_new;
+          const float p0 = exp2f(sc[r][0] - m_use), p1 = exp2f(sc[r][1] - m_use);
+          const float p2 = exp2f(sc[r][2] - m_use), p3 = exp2f(sc[r][3] - m_use);
+          l_run[r] = l_run[r] * alpha[r] + ((p0 + p1) + (p2 + p3));
+          pa[r] = pack2<T>(p0, p1);        // A fragment: row gid (+8), keys 2tig, 2tig+1
+          pa[2 + r] = pack2<T>(p2, p3);    //             row gid (+8), keys 8+2tig, 9+2tig
+        }
+        if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+          for (int i = 0; i < NDT; ++i) {
+            acc[i][0] *= alpha[0]; acc[i][1] *= alpha[0];
+            acc[i][2] *= alpha[1]; acc[i][3] *= alpha[1];
+          }
+        }
+        // ---- O[g, d] += P V
+        {
+          const int mi = lane >> 3, r = lane & 7;
+          const int row = 16 * warp + 8 * (mi & 1) + r;
+#pragma unroll
+          for (int dp = 0; dp < NDT / 2; ++dp) {
+            const int c16 = 2 * dp + (mi >> 1);
+            const uint32_t addr = vtile + (c16 >> 3) * L::kPanelBytes + row * 128 + (((c16 & 7) ^ (row & 7)) << 4);
+            unsigned b0, b1, b2, b3;
+            ldmatrix_x4_trans(addr, b0, b1, b2, b3);
+            mma_16816<T>(acc[2 * dp], pa[0], pa[1], pa[2], pa[3], b0, b1);
+            mma_16816<T>(acc[2 * dp + 1], pa[0], pa[1], pa[2], pa[3], b2, b3);
           }
         }
       }
-      const unsigned vmask = __ballot_sync(0xffffffffu, ok) & 0xffffu;
-      if (vmask != 0xffffu) {
-        // rows of V that are not real keys may hold anything (cache padding): P = 0
-        // times NaN would poison O, so they are cleared in shared memory first
-        uint8_t* vgen = sgen + (vtile - sbase);
-        for (int r = 0; r < 16; ++r) {
-          if ((vmask >> r) & 1u) continue;
-          const int row = 16 * warp + r;
-          for (int i = lane; i < L::kPanels * 8; i += 32)
-            *reinterpret_cast<uint4*>(vgen + (i >> 3) * L::kPanelBytes + row * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
-        }
-        fence_proxy_async();   // these plain stores precede the copy engine's next write to the stage
-        __syncwarp();
-      }
-      // ---- S[g, key] = Q K^T for two 8-key tiles
-      float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-      {
-        const int mi = lane >> 3, r = lane & 7;
-        const int row = 16 * warp + 8 * (mi >> 1) + r;
-#pragma unroll
-        for (int kt = 0; kt < NKT; ++kt) {
-          const int c16 = 2 * kt + (mi & 1);
-          const uint32_t addr = ktile + (c16 >> 3) * L::kPanelBytes + row * 128 + (((c16 & 7) ^ (row & 7)) << 4);
-          unsigned b0, b1, b2, b3;
-          ldmatrix_x4(addr, b0, b1, b2, b3);
-          mma_16816<T>(c0, qa[kt][0], qa[kt][1], qa[kt][2], qa[kt][3], b0, b1);
-          mma_16816<T>(c1, qa[kt][0], qa[kt][1], qa[kt][2], qa[kt][3], b2, b3);
-        }
-      }
-      // columns of this thread: keys 2tig, 2tig+1 (c0) and 8+2tig, 9+2tig (c1); rows gid (x0,x1) and gid+8 (x2,x3)
-      float sc[2][4];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        sc[r][0] = ((vmask >> (2 * tig)) & 1u) ? c0[2 * r] * p.scale_log2 : -INFINITY;
-        sc[r][1] = ((vmask >> (2 * tig + 1)) & 1u) ? c0[2 * r + 1] * p.scale_log2 : -INFINITY;
-        sc[r][2] = ((vmask >> (8 + 2 * tig)) & 1u) ? c1[2 * r] * p.scale_log2 : -INFINITY;
-        sc[r][3] = ((vmask >> (9 + 2 * tig)) & 1u) ? c1[2 * r + 1] * p.scale_log2 : -INFINITY;
-      }
-      float alpha[2];
-      unsigned pa[4];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        float mx = fmaxf(fmaxf(sc[r][0], sc[r][1]), fmaxf(sc[r][2], sc[r][3]));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float m_new = fmaxf(m_run[r], mx);
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        alpha[r] = exp2f(m_run[r] - m_use);
-        m_run[r] = m_new;
-        const float p0 = exp2f(sc[r][0] - m_use), p1 = exp2f(sc[r][1] - m_use);
-        const float p2 = exp2f(sc[r][2] - m_use), p3 = exp2f(sc[r][3] - m_use);
-        l_run[r] = l_run[r] * alpha[r] + ((p0 + p1) + (p2 + p3));
-        pa[r] = pack2<T>(p0, p1);        // A fragment: row gid (+8), keys 2tig, 2tig+1
-        pa[2 + r] = pack2<T>(p2, p3);    //             row gid (+8), keys 8+2tig, 9+2tig
-      }
-      if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-        for (int i = 0; i < NDT; ++i) {
-          acc[i][0] *= alpha[0]; acc[i][1] *= alpha[0];
-          acc[i][2] *= alpha[1]; acc[i][3] *= alpha[1];
-        }
-      }
-      // ---- O[g, d] += P V
-      {
-        const int mi = lane >> 3, r = lane & 7;
-        const int row = 16 * warp + 8 * (mi & 1) + r;
-#pragma unroll
-        for (int dp = 0; dp < NDT / 2; ++dp) {
-          const int c16 = 2 * dp + (mi >> 1);
-          const uint32_t addr = vtile + (c16 >> 3) * L::kPanelBytes + row * 128 + (((c16 & 7) ^ (row & 7)) << 4);
-          unsigned b0, b1, b2, b3;
-          ldmatrix_x4_trans(addr, b0, b1, b2, b3);
-          mma_16816<T>(acc[2 * dp], pa[0], pa[1], pa[2], pa[3], b0, b1);
-          mma_16816<T>(acc[2 * dp + 1], pa[0], pa[1], pa[2], pa[3], b2, b3);
-        }
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty(s));
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty(s));
-  }
 
-  // ---- combine the four warps (the ring is free now: every stage was consumed)
+    // ---- fold the four warps' sums, 32 or 64 columns at a time, through a buffer beside the ring (the
+    // producer is already filling the ring for the next item)
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
-  }
-  asm volatile("bar.sync 1, 128;" ::: "memory");
-  const int heads_here = min(16, p.group - gg * 16);
-  const int D = p.head_dim_rt;
-  if (*abort_flag) {
-    // A bounded wait gave up (flash_attn_decoding.py has no counterpart: its loads cannot
-    // stall).  The ring may still be receiving copies, so it is not reused as the combine
-    // buffer: the chunk is reported as empty and the caller is told through the status word.
-    for (int idx = threadIdx.x; idx < heads_here * D; idx += 128) {
-      const int g = idx / D, d = idx - g * D;
-      const long long row = ((long long)b * p.heads_q + hk * p.group + gg * 16 + g) * p.max_chunks + chunk_id;
-      p.part_o[row * D + d] = 0.f;
-      if (d == 0) p.part_lse[row] = -INFINITY;
+    for (int r = 0; r < 2; ++r) {
+      l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
+      l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
     }
-    if (threadIdx.x == 0 && p.status_word) atomicExch(p.status_word, 1);
-    return;
-  }
-  float* sm_o = reinterpret_cast<float*>(sgen);                       // [4][16][DP + 1]
-  float* sm_m = sm_o + 4 * 16 * L::kCombinePitch;                      // [4][16]
-  float* sm_l = sm_m + 4 * 16;
-  if (tig == 0) {
-    sm_m[warp * 16 + gid] = m_run[0]; sm_m[warp * 16 + gid + 8] = m_run[1];
-    sm_l[warp * 16 + gid] = l_run[0]; sm_l[warp * 16 + gid + 8] = l_run[1];
-  }
-#pragma unroll
-  for (int i = 0; i < NDT; ++i) {
-    float* r0 = sm_o + (warp * 16 + gid) * L::kCombinePitch + 8 * i + 2 * tig;
-    float* r1 = sm_o + (warp * 16 + gid + 8) * L::kCombinePitch + 8 * i + 2 * tig;
-    r0[0] = acc[i][0]; r0[1] = acc[i][1];
-    r1[0] = acc[i][2]; r1[1] = acc[i][3];
-  }
-  asm volatile("bar.sync 1, 128;" ::: "memory");
-  for (int idx = threadIdx.x; idx < heads_here * D; idx += 128) {
-    const int g = idx / D, d = idx - g * D;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, sm_m[w * 16 + g]);
-    const float Ms = (M == -INFINITY) ? 0.f : M;
-    float Lsum = 0.f, O = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float f = exp2f(sm_m[w * 16 + g] - Ms);
-      Lsum += sm_l[w * 16 + g] * f;
-      O += sm_o[(w * 16 + g) * L::kCombinePitch + d] * f;
+    if (tig == 0) {
+      sm_m[warp * 16 + gid] = m_run[0]; sm_m[warp * 16 + gid + 8] = m_run[1];
+      sm_l[warp * 16 + gid] = l_run[0]; sm_l[warp * 16 + gid + 8] = l_run[1];
     }
-    const int hq = hk * p.group + gg * 16 + g;
-    const long long row = ((long long)b * p.heads_q + hq) * p.max_chunks + chunk_id;
-    p.part_o[row * D + d] = Lsum > 0.f ? O / Lsum : 0.f;
-    if (d == 0) p.part_lse[row] = Lsum > 0.f ? Ms + log2f(Lsum) : -INFINITY;
+    bool gave_up = false;
+    auto fold = [&](auto rows_c) {
+      constexpr int kRows = decltype(rows_c)::value;      // MMA rows that hold heads: 8 or 16
+      constexpr int kCols = 32 * (16 / kRows), kPitch = kCols + 1;
+#pragma unroll
+      for (int rd = 0; rd < DP / kCols; ++rd) {
+#pragma unroll
+        for (int i = 0; i < kCols / 8; ++i) {
+          const float* a4 = acc[(kCols / 8) * rd + i];
+          float* r0 = sm_fold + (warp * kRows + gid) * kPitch + 8 * i + 2 * tig;
+          r0[0] = a4[0]; r0[1] = a4[1];
+          if (kRows == 16) { r0[8 * kPitch] = a4[2]; r0[8 * kPitch + 1] = a4[3]; }
+        }
+        // (a bounded wait gave up: the chunk is reported as empty and the caller is told through the
+        // status word; flash_attn_decoding.py has no counterpart, its loads cannot stall)
+        gave_up = consumers_any(*abort_flag != 0) || gave_up;
+        for (int g = warp; g < heads_here; g += 4) {
+          float M = -INFINITY;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) M = fmaxf(M, sm_m[w * 16 + g]);
+          const float Ms = (M == -INFINITY) ? 0.f : M;
+          float f[4], Lsum = 0.f;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            f[w] = exp2f(sm_m[w * 16 + g] - Ms);
+            Lsum += sm_l[w * 16 + g] * f[w];
+          }
+          const bool some = Lsum > 0.f && !gave_up;
+          const int hq = hk * p.group + gg * 16 + g;
+          const long long prow = ((long long)b * p.heads_q + hq) * p.max_chunks + chunk_id;
+#pragma unroll
+          for (int cc = 0; cc < kCols; cc += 32) {
+            float O = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) O += sm_fold[(w * kRows + g) * kPitch + cc + lane] * f[w];
+            const float v = some ? O / Lsum : 0.f;
+            const int d = kCols * rd + cc + lane;
+            if (d < D) {
+              if (p.direct_o) ((T*)p.o)[(long long)b * p.o_sb + (long long)hq * p.o_sh + d] = from_float<T>(v);
+              else p.part_o[prow * D + d] = v;
+            }
+          }
+          if (rd == 0 && lane == 0 && !p.direct_o) p.part_lse[prow] = some ? Ms + log2f(Lsum) : -INFINITY;
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      }
+    };
+    if (p.group <= 8) fold(std::integral_constant<int, 8>());
+    else fold(std::integral_constant<int, 16>());
+    if (gave_up) break;
   }
+  if (threadIdx.x == 0 && *abort_flag && p.status_word) atomicExch(p.status_word, 1);
 }
 
 // Phase 2: O = sum_c o_c * 2^(lse_c - lse), lse = log2 sum_c 2^lse_c
 // (flash_attn_decoding.py:173-208).  Sequences without visible keys give 0.
+// A few KB per CTA, so its time is the number of dependent memory round trips: the chunk LSEs are
+// read a chunk per lane, the chunk rows four at a time per warp (a warp per fourth chunk, a
+// 16-byte load per lane), and the warps' sums meet in shared memory.
+constexpr int kCombineWarps = 4;
+
 template <typename T, int D>
-__global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(32 * kCombineWarps) decode_combine_kernel(const DecodeParams p) {
   // Launched with programmatic stream serialisation: its CTAs may be set up while phase 1 is
   // still draining, and wait here until that whole grid has finished and its partials are
   // visible (a no-op when launched the ordinary way).
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  sm100::grid_dependency_wait();
+  constexpr int kLanes = D / 4;                     // lanes that hold 4 columns each
   const int hq = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const KeyMap km = make_keymap(p, b, hq / p.group);
   const int nchunk = (km.n + p.chunk - 1) / p.chunk;
   const long long row0 = ((long long)b * p.heads_q + hq) * p.max_chunks;
+  const float* lse = p.part_lse + row0;
   float M = -INFINITY;
-  for (int c = 0; c < nchunk; ++c) M = fmaxf(M, p.part_lse[row0 + c]);
+  for (int c = lane; c < nchunk; c += 32) M = fmaxf(M, lse[c]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   const float Ms = (M == -INFINITY) ? 0.f : M;
   float L = 0.f;
-  for (int c = 0; c < nchunk; ++c) L += exp2f(p.part_lse[row0 + c] - Ms);
+  for (int c = lane; c < nchunk; c += 32) L += exp2f(lse[c] - Ms);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
   const float inv = L > 0.f ? 1.f / L : 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (lane < kLanes) {
+    const float4* rows = reinterpret_cast<const float4*>(p.part_o + row0 * D) + lane;
+#pragma unroll 4
+    for (int c = warp; c < nchunk; c += kCombineWarps) {
+      const float w = exp2f(lse[c] - Ms) * inv;
+      const float4 r = rows[(long long)c * kLanes];
+      acc.x = fmaf(r.x, w, acc.x); acc.y = fmaf(r.y, w, acc.y);
+      acc.z = fmaf(r.z, w, acc.z); acc.w = fmaf(r.w, w, acc.w);
+    }
+  }
+  __shared__ float4 part[kCombineWarps][kLanes];
+  if (lane < kLanes) part[warp][lane] = acc;
+  __syncthreads();
   T* orow = (T*)p.o + (long long)b * p.o_sb + (long long)hq * p.o_sh;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float acc = 0.f;
-    for (int c = 0; c < nchunk; ++c)
-      acc += p.part_o[(row0 + c) * D + d] * (exp2f(p.part_lse[row0 + c] - Ms) * inv);
-    orow[d] = from_float<T>(acc);
+  const int d = threadIdx.x;
+  if (d < D) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kCombineWarps; ++w) s += reinterpret_cast<const float*>(part[w])[d];
+    orow[d] = from_float<T>(s);
   }
 }
 
@@ -659,24 +835,48 @@ static int decode_max_visible(const b200attn_decode_args* a) {
   return a->max_seqlen;
 }
 
-// Split size.  A CTA has a fixed cost (length lookup, Q load, pipeline fill, cross-warp
-// combine: ~2.8 us), so longer chunks move more bytes per CTA, but the launch still has
-// to fill the machine and ragged batches need several CTAs per slot to balance.  Measured
-// on B200 (bf16, D = 128, GB/s of KV):
-//   many units (batch x KV heads x 16-query-head groups >= 256): 2048 keys is best or within
-//     1 % of best (config 3, ragged: 6290 at 2048, 6120 at 4096, 5560 at 8192; config 5: 6110
-//     at 2048, 5600 at 4096);
-//   few units: the longest power-of-two chunk that still gives one CTA per SM (batch 8 x 32768
-//     keys: 6630 at 8192, 5870 at 1024; batch 1 x 131072: 5900 at 4096, 3270 at 512; batch 4, 128
-//     query heads: 4650 at 2048, 2140 at 256; batch 3 x 20000: 4980 at 2048, 4310 at 1024).
-//     Chunks cut to fill exactly one wave of 296 CTAs (e.g. 3584 keys) measured 4-7 % slower
-//     than the neighbouring power of two.
+// Split size.  A chunk has a fixed cost (its set-up where that is not hidden, the fold, its partial
+// rows), so longer chunks move more bytes per unit of it, but the launch has to fill the machine
+// (two CTAs per SM) and ragged batches need several chunks per CTA to balance.  A unit is a
+// (sequence, KV head, 16 query heads).  Measured on B200 (bf16, D = 128; us of phases 1 and 2):
+//   block lists and windows (every unit has about the same number of keys): the number of chunks
+//     with the least waves x (stages of a chunk + 3), a chunk's fixed cost being ~3 stages.  256
+//     units x 4096 keys: 86.5 in one chunk, 90.6 in two, 93.0 in four; 512 x 2112: 87.4 / 92.4;
+//     16 x 2560: 12.7 in 192-key chunks, 14.2 in 512.
+//   lengths up to max_seqlen, 256 units or more: 2048 keys is best or within 1 % of best (64
+//     sequences x 8 heads, 1024-8192 keys: 187.5; 188.8 at 1024, 194 at 4096).
+//   64 to 255 units: 1024 keys up to 8192, 2048 beyond (192 units, 300-6000 keys in pages of 64: 62.9,
+//     70.6 in one chunk each; 64 units, 200-30000 keys: 87.9, 100 at 8192; 128 units, 2000-16000:
+//     120.7, 135 at 4096, 118.9 at 8192).
+//   fewer: the longest power-of-two chunk that still gives one CTA per SM (8 units x 131072 keys:
+//     5900 GB/s at 4096, 3270 at 512).
+constexpr int kDecodeSlots = 2 * 148;
+static size_t partial_bytes(const b200attn_decode_args* a, long long chunks) {
+  const long long rows = (long long)a->batch * a->heads_q * (chunks < 1 ? 1 : chunks);
+  return (size_t)(rows * a->head_dim * 4 + rows * 4);
+}
 static int decode_chunk(const b200attn_decode_args* a) {
   if (a->chunk_tokens > 0) return a->chunk_tokens;
   const long long group = a->heads_kv > 0 ? a->heads_q / a->heads_kv : 1;
   const long long units = (long long)a->batch * a->heads_kv * ((group + 15) / 16);
   const long long visible = decode_max_visible(a);
+  if (a->sparsity == B200ATTN_BLOCK_LIST || a->sparsity == B200ATTN_WINDOW) {
+    const long long stages = visible > 0 ? (visible + 63) / 64 : 1;
+    long long best = 1, best_cost = -1;
+    for (long long c = 1; c <= stages && c <= 128; ++c) {
+      const long long per = (stages + c - 1) / c;
+      const long long cost = ((units * c + kDecodeSlots - 1) / kDecodeSlots) * (per + 3);
+      if (best_cost < 0 || cost < best_cost) { best = per; best_cost = cost; }
+    }
+    return (int)(64 * best);
+  }
   if (units >= 256) return 2048;
+  if (units >= 64) {
+    // (no more scratch than the module's fixed array has, where longer chunks avoid that)
+    int c = visible <= 8192 ? 1024 : 2048;
+    while (c < 8192 && partial_bytes(a, (visible + c - 1) / c) > (size_t)B200ATTN_NOALLOC_SCRATCH_BYTES) c *= 2;
+    return c;
+  }
   const int sizes[7] = {8192, 4096, 2048, 1024, 512, 256, 128};
   for (int c : sizes)
     if (units * ((visible + c - 1) / c) >= 148) return c;   // at least one CTA per SM
@@ -686,10 +886,7 @@ static int decode_chunk(const b200attn_decode_args* a) {
 size_t decode_workspace_bytes(const b200attn_decode_args* a) {
   if (!a || a->batch <= 0 || a->heads_q <= 0 || a->head_dim <= 0) return 0;
   int chunk = decode_chunk(a);
-  long long chunks = (decode_max_visible(a) + chunk - 1) / chunk;
-  if (chunks < 1) chunks = 1;
-  long long rows = (long long)a->batch * a->heads_q * chunks;
-  return (size_t)(rows * a->head_dim * 4 + rows * 4);
+  return partial_bytes(a, (decode_max_visible(a) + chunk - 1) / chunk);
 }
 
 static int validate_decode(const b200attn_decode_args* a, bool sparse, bool paged) {
@@ -729,17 +926,7 @@ static int validate_decode(const b200attn_decode_args* a, bool sparse, bool page
 // which counts when the whole decoding step is a few tens of microseconds.
 template <typename T, int D>
 static cudaError_t launch_combine(const DecodeParams& p, dim3 g2, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g2;
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, decode_combine_kernel<T, D>, p);
+  return launch_after(decode_combine_kernel<T, D>, g2, dim3(32 * kCombineWarps), 0, stream, p);
 }
 
 template <typename T, int D>
@@ -775,15 +962,15 @@ static DecEncodeFn dec_encode_fn() {
   }();
   return fn;
 }
-// [D, keys, kv heads, batch] view of a cache, box = 64 x 16 x 1 x 1, 128-byte swizzle
+// [D, keys, kv heads, batch] view of a cache, box = 64 x box_keys x 1 x 1, 128-byte swizzle
 static bool make_cache_tmap(CUtensorMap* m, int dtype, const void* base, int D, long long keys, int heads, int batch,
-                            long long st, long long sh, long long sb) {
+                            long long st, long long sh, long long sb, int box_keys) {
   DecEncodeFn enc = dec_encode_fn();
   if (!enc) return false;
   if (batch <= 1 || sb <= 0) sb = st * keys;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)keys, (cuuint64_t)heads, (cuuint64_t)batch};
   cuuint64_t strides[3] = {(cuuint64_t)st * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
-  cuuint32_t box[4] = {64, (cuuint32_t)kBoxTok, 1, 1};
+  cuuint32_t box[4] = {64, (cuuint32_t)box_keys, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   return enc(m, dtype == B200ATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
              const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -800,14 +987,24 @@ static int launch_decode_tma_d(const b200attn_decode_args* a, const DecodeParams
   // tensor maps: it makes the device's context current on this thread, which their encoder needs)
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
     return B200ATTN_ERR_CUDA;
-  CUtensorMap tk, tv;
-  if (!make_cache_tmap(&tk, a->dtype, a->k_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch,
-                       a->k_stride_t, a->k_stride_h, a->k_stride_b) ||
-      !make_cache_tmap(&tv, a->dtype, a->v_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch,
-                       a->v_stride_t, a->v_stride_h, a->v_stride_b))
+  // single 16-key boxes for gathers and chunk ends, whole 64-key stages where the keys are consecutive
+  CUtensorMap tk, tv, tk64, tv64;
+  auto key_map = [&](CUtensorMap* m, int box) {
+    return make_cache_tmap(m, a->dtype, a->k_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch, a->k_stride_t,
+                           a->k_stride_h, a->k_stride_b, box);
+  };
+  auto value_map = [&](CUtensorMap* m, int box) {
+    return make_cache_tmap(m, a->dtype, a->v_cache, a->head_dim, p.map_keys, a->heads_kv, p.map_batch, a->v_stride_t,
+                           a->v_stride_h, a->v_stride_b, box);
+  };
+  if (!key_map(&tk, kBoxTok) || !value_map(&tv, kBoxTok) || !key_map(&tk64, kStageTok) || !value_map(&tv64, kStageTok))
     return B200ATTN_ERR_CUDA;
-  kern<<<g1, 160, L::kAlloc, stream>>>(tk, tv, p);
-  cudaError_t e;
+  cudaError_t e = launch_after(kern, g1, dim3(160), L::kAlloc, stream, tk, tv, tk64, tv64, p);
+  if (e != cudaSuccess) return B200ATTN_ERR_CUDA;
+  if (p.direct_o) {
+    set_launch_count(1);
+    return e == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
+  }
   switch (a->head_dim) {
     case 32: e = launch_combine<T, 32>(p, g2, stream); break;
     case 64: e = launch_combine<T, 64>(p, g2, stream); break;
@@ -838,7 +1035,8 @@ static int decode_fwd_impl(const b200attn_decode_args* a, bool sparse, long long
   size_t need = decode_workspace_bytes(&eff);
   if (!ws || ws_bytes < need) return scratch ? B200ATTN_ERR_TOO_LARGE : B200ATTN_ERR_WORKSPACE;
   if ((uintptr_t)ws & 15) return B200ATTN_ERR_ALIGN;
-  st = device_info(nullptr);
+  const DeviceInfo* di = nullptr;
+  st = device_info(&di);
   if (st != B200ATTN_OK) return st;
 
   DecodeParams p;
@@ -862,6 +1060,7 @@ static int decode_fwd_impl(const b200attn_decode_args* a, bool sparse, long long
   p.head_dim_rt = a->head_dim;
   p.max_seqlen = a->max_seqlen;
   p.status_word = a->status_word;
+  p.direct_o = p.take_over = 0;
   // keys beyond max_seqlen are never visible; the copy engine zero-fills past the extent
   p.map_keys = pool_keys > 0 ? pool_keys : a->max_seqlen;
   p.map_batch = pool_keys > 0 ? 1 : a->batch;
@@ -877,7 +1076,9 @@ static int decode_fwd_impl(const b200attn_decode_args* a, bool sparse, long long
                       a->max_seqlen > 0;
   if (tma_ok) {
     p.ggroups = (p.group + 15) / 16;
-    dim3 g1t(a->heads_kv * p.ggroups, p.max_chunks, a->batch);
+    p.direct_o = p.max_chunks == 1;
+    p.take_over = (long long)a->heads_kv * p.ggroups * a->batch * p.max_chunks > 2LL * di->sm_count;
+    dim3 g1t(a->heads_kv * p.ggroups, a->batch, p.max_chunks);
     return a->dtype == B200ATTN_F16 ? launch_decode_tma<__half>(a, p, g1t, g2, stream)
                                     : launch_decode_tma<__nv_bfloat16>(a, p, g1t, g2, stream);
   }

@@ -5,6 +5,7 @@
 // flash_attn_triton/flash_attn_decoding_sparse.py:445-466).  Pure byte moves:
 // 16-byte vector copies, one warp per (token, head) row, bound by HBM.
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace b200attn {
 namespace {
@@ -38,6 +39,9 @@ __global__ void append_kernel(const uint4* __restrict__ new_k, const uint4* __re
                               const int32_t* __restrict__ seqlens, long long n_sb, long long n_sh,
                               long long c_sb, long long c_st, long long c_sh, int batch, int capacity,
                               int heads, int vec_per_row) {
+  // (a decoding kernel behind this one is set up meanwhile, as this one is behind the step before)
+  sm100::launch_dependents();
+  sm100::grid_dependency_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= (long long)batch * heads) return;
   const int lane = threadIdx.x & 31;
@@ -88,10 +92,11 @@ int kv_append(const b200attn_kv_append_args* a, cudaStream_t stream) {
   const long long rows = (long long)a->batch * a->heads;
   const int wpb = 8;
   if (int dst = device_info(nullptr)) return dst;
-  append_kernel<<<(unsigned)((rows + wpb - 1) / wpb), wpb * 32, 0, stream>>>(
+  if (launch_after(append_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32), 0, stream,
       (const uint4*)a->new_k, (const uint4*)a->new_v, (uint4*)a->k_cache, (uint4*)a->v_cache, a->seqlens,
       a->new_stride_b / 8, a->new_stride_h / 8, a->cache_stride_b / 8, a->cache_stride_t / 8,
-      a->cache_stride_h / 8, a->batch, a->capacity, a->heads, a->head_dim / 8);
+      a->cache_stride_h / 8, a->batch, a->capacity, a->heads, a->head_dim / 8) != cudaSuccess)
+    return B200ATTN_ERR_CUDA;
   set_launch_count(1);
   return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
 }

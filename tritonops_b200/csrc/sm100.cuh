@@ -31,6 +31,32 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ------------------------------------------------------- cluster launch control
+// Ask for a CTA of this grid that has not been launched yet, to do its work instead of it: the
+// 16-byte answer lands at `dst` (shared, 16-byte aligned) and completes 16 bytes on `bar`.  After an
+// answer that no CTA was left, nothing may be asked again.
+__device__ __forceinline__ void try_cancel_next_cta(uint32_t dst, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(dst), "r"(bar)
+               : "memory");
+}
+// The answer: true and the coordinates of the CTA that was taken over, or false.
+__device__ __forceinline__ bool next_cta(uint32_t answer, int& x, int& y, int& z) {
+  uint32_t ok, cx, cy, cz;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 r, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %3, 1, 0, p;\n\t"
+      "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n\t}"
+      : "=&r"(cx), "=&r"(cy), "=&r"(cz), "=&r"(ok)
+      : "r"(answer)
+      : "memory");
+  if (ok) { x = (int)cx; y = (int)cy; z = (int)cz; }
+  return ok != 0;
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
