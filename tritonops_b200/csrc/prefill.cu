@@ -3,8 +3,9 @@
 // Stands in for flash_attn_fwd_kernel (flash_attn_triton/flash_attn_triton.py:52-180)
 // and its window twin (flash_attn_triton/flash_attn_sparse_attn_triton.py:47-234).
 //
-// One CTA owns 256 consecutive query rows of one (sequence, query head) as two
-// 128-row tiles and walks the visible KV tiles once for both:
+// A work item is 256 consecutive query rows of one (sequence, query head): a CTA holds
+// them as two 128-row tiles and walks the visible KV tiles once for both (one item per
+// CTA, or for packed launches and windows items taken over until none is left):
 //
 //   warp 9   TMA producer: Q_0, K_0, Q_1, then V_0, K_1, V_1, ... into a ring of
 //            128-byte-swizzled shared-memory stages (mbarrier full/empty pairs)
@@ -15,11 +16,12 @@
 //            registers (base-2 exponentials), writes P back over S as packed
 //            16-bit values for the P V product, rescales O in TMEM only when
 //            the row max has grown by more than 2^8, and writes the output (a
-//            tile inside its sequence through the dead Q buffer and a TMA store).
+//            tile inside its sequence through shared memory and a TMA store).
 //
 // While one warpgroup computes the softmax of its tile the tensor core works on
 // the other tile, so MMA and exponentials overlap.  TMEM columns: S0 [0,128),
-// S1 [128,256), O0 [256,256+D), O1 [384,384+D); P_t aliases the first half of S_t.
+// S1 [128,256), O0 [256,256+D), O1 behind it; P_t lies over the first half of S_t with
+// 128-wide heads, and in columns of its own from 384 with narrower ones.
 // Every mbarrier wait is bounded; a timeout sets *status_word and the CTA drains.
 #include <mutex>
 #include <algorithm>
@@ -198,30 +200,57 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-template <int DP, int BN, int NSTAGE>
+// One work item (256 query rows of one sequence and head) as the loader hands it to the other roles.
+struct PrefillItem {
+  int q0, h, b;           // first query row, query head, sequence
+  int seq_start, len;     // where the sequence starts in packed tensors, its length
+  int valid;              // 0: no more items
+};
+
+// What a CTA works on: one item found from its coordinates, items handed out until none is left, or
+// one item with block-list sparsity (own instantiations, so that none carries the others' branches).
+enum PrefillMode { kOneItem, kManyItems, kBlockList };
+
+template <int DP, int BN, int NSTAGE, PrefillMode MODE>
 struct PrefillSmem {
   static constexpr int kQBytes = kTileM * DP * 2;
   static constexpr int kQPanel = kTileM * 128;  // one 64-column swizzled panel of Q
   static constexpr int kStageBytes = BN * DP * 2;
   static constexpr int kKvPanel = BN * 128;
-  static constexpr int kBarOffset = 2 * kQBytes + NSTAGE * kStageBytes;
-  static constexpr int kNumBars = 2 + 2 * NSTAGE + 8;
+  static constexpr int kOut = 2 * kQBytes + NSTAGE * kStageBytes;    // (many items) an output tile on its way out
+  static constexpr int kBarOffset = kOut + (MODE == kManyItems ? kQBytes : 0);
+  static constexpr int kNumBars = 2 + 2 * NSTAGE + 8 + 6;
   // block-list mode: 4 bitmaps (one per 64-row query block of the CTA), then per
   // query tile the merged ascending list of KV blocks with a 2-bit membership mask
-  static constexpr int kBitmapOffset = kBarOffset + kNumBars * 8 + 16;
+  static constexpr int kItem = kBarOffset + kNumBars * 8 + 16;
+  static constexpr int kNext = (kItem + 24 + 15) / 16 * 16;          // answer of the launch control
+  static constexpr int kBitmapOffset = kNext + 16;
   static constexpr int kUlistOffset = kBitmapOffset + 4 * (kMaxBlocks / 32) * 4;
   static constexpr int kUflagOffset = kUlistOffset + 2 * kMaxBlocks * 2;
-  static constexpr int kBytes = kUflagOffset + 2 * kMaxBlocks;
+  static constexpr int kBytes = MODE == kBlockList ? kUflagOffset + 2 * kMaxBlocks : kBitmapOffset;
   static constexpr int kAlloc = kBytes + 1024;  // slack to align the base to 1024 bytes
+  static_assert(kAlloc <= 232448, "shared memory of one CTA");
 };
 
-// BLK: block-list sparsity (own instantiation so the dense / window paths carry none of its branches)
-template <typename T, int DP, int BN, int NSTAGE, bool BLK>
+// barrier of 128 threads; true if `flag` is for any of them
+__device__ __forceinline__ bool group_any(int id, bool flag) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(flag ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
+template <typename T, int DP, int BN, int NSTAGE, PrefillMode MODE>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
                const PrefillParams p) {
-  using L = PrefillSmem<DP, BN, NSTAGE>;
+  using L = PrefillSmem<DP, BN, NSTAGE, MODE>;
+  constexpr bool BLK = MODE == kBlockList, MANY = MODE == kManyItems;
   constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   constexpr uint32_t kIdescQK = idesc_f16(kFmt, false, kTileM, BN);
   constexpr uint32_t kIdescPV = idesc_f16(kFmt, true, kTileM, DP);
@@ -251,6 +280,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   auto p_full = [&](int t) { return bars + 8 * (4 + 2 * NSTAGE + t); };
   auto o_full = [&](int t) { return bars + 8 * (6 + 2 * NSTAGE + t); };
   auto s_free = [&](int t) { return bars + 8 * (8 + 2 * NSTAGE + t); };
+  auto q_free = [&](int t) { return bars + 8 * (10 + 2 * NSTAGE + t); };
+  const uint32_t item_full = bars + 8 * (12 + 2 * NSTAGE), item_empty = item_full + 8, next_full = item_full + 16,
+                 out_free = item_full + 24;
+  volatile PrefillItem* item = reinterpret_cast<volatile PrefillItem*>(smem_gen + L::kItem);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kBarOffset + L::kNumBars * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + L::kBarOffset + L::kNumBars * 8 + 4);
 
@@ -263,7 +296,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       mbar_init(p_full(t), 4);
       mbar_init(o_full(t), 1);
       mbar_init(s_free(t), 4);
+      mbar_init(q_free(t), 1);
     }
+    mbar_init(item_full, 1);
+    mbar_init(item_empty, 9);      // the MMA warp and eight softmax warps
+    mbar_init(next_full, 1);
+    mbar_init(out_free, 1);
     for (int s = 0; s < NSTAGE; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
     fence_barrier_init();
     fence_proxy_async();
@@ -295,19 +333,45 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     h_ = bh % p.heads_q; b_ = bh / p.heads_q;
     return true;
   };
-  int b, h, pair;
-  if (!locate(blockIdx.x, b, h, pair)) return;
-  const int hk = h / p.group;
-  int seq_start = 0, len = p.seqlen, bcoord = b;
-  if (p.cu_seqlens) {
-    seq_start = p.cu_seqlens[b];
-    // a sequence longer than the max_seqlen the grid was sized for is cut there
-    len = min(p.cu_seqlens[b + 1] - seq_start, p.n_pairs * kPairM);
-    bcoord = 0;
+  // The item at hand, for each role its own: taken from the CTA's coordinates, or (many items) handed
+  // over by the loader.
+  int b = 0, h = 0, hk = 0, seq_start = 0, len = 0, bcoord = 0, q0 = 0;
+  TileSeq seq = {0, 0, 0};
+  auto place = [&](int b_, int h_, int pair_) {     // false: nothing there
+    b = b_; h = h_; hk = h / p.group;
+    q0 = pair_ * kPairM;
+    seq_start = 0; len = p.seqlen; bcoord = b;
+    if (p.cu_seqlens) {
+      seq_start = p.cu_seqlens[b];
+      // a sequence longer than the max_seqlen the grid was sized for is cut there
+      len = min(p.cu_seqlens[b + 1] - seq_start, p.n_pairs * kPairM);
+      bcoord = 0;
+    }
+    if (q0 >= len) return false;
+    seq = make_seq<BN>(p, q0, len);
+    return true;
+  };
+  if (!MANY) {
+    int b_, h_, pair_;
+    if (!locate(blockIdx.x, b_, h_, pair_) || !place(b_, h_, pair_)) return;
   }
-  const int q0 = pair * kPairM;
-  if (q0 >= len) return;
-  const TileSeq seq = make_seq<BN>(p, q0, len);
+  // The next item the loader has handed over (n: how many this role has had); false when there is
+  // none.  `all`: makes the answer of the wait the same for all threads of the role (after a wait
+  // gave up, one might see its phase complete and another the abort flag).
+  auto next_item = [&](int n, auto all) -> bool {
+    if (!MANY) return n == 0;
+    const bool got = mbar_wait(item_full, n & 1, abort_flag);
+    if (!all(got)) return false;
+    const bool valid = item->valid != 0;
+    q0 = item->q0; h = item->h; b = item->b; seq_start = item->seq_start; len = item->len;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(item_empty);
+    if (!valid) return false;
+    hk = h / p.group;
+    bcoord = p.cu_seqlens ? 0 : b;
+    seq = make_seq<BN>(p, q0, len);
+    return true;
+  };
 
   if (warp == 0) {
     __syncwarp();
@@ -387,7 +451,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   // steps of each tile in block-list mode (its own K/V stream), else of the CTA
   const int ns0 = (q0 < len) ? (n_u[0] + 1) / 2 : 0;
   const int ns1 = (q0 + kTileM < len) ? (n_u[1] + 1) / 2 : 0;
-  const int n_steps = blk ? max(ns0, ns1) : seq.n;
   // does query tile t take part in step j?
   auto step_active = [&](int t, int j) -> bool {
     if (!blk) return tile_active<BN>(p, q0 + kTileM * t, len, seq.kv(j));
@@ -401,8 +464,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // ================================================================= TMA
     {
       if (elect_one()) { prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_o); }
+      int q_loads[2] = {0, 0};
       auto load_q = [&](int t) {
         if (q0 + kTileM * t >= len) return;
+        // (the products of the item before have read the tile)
+        if (q_loads[t] > 0) mbar_wait(q_free(t), (q_loads[t] - 1) & 1, abort_flag);
+        ++q_loads[t];
         if (elect_one()) {
           mbar_expect_tx(q_full(t), L::kQBytes);
           for (int pn = 0; pn < kPanels; ++pn)
@@ -411,8 +478,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
         __syncwarp();
       };
-      load_q(0);
-      // The CTA that will start when one of the resident ones ends finds its Q tiles (read by
+      // (One item) the CTA that will start when one of the resident ones ends finds its Q tiles (read by
       // nobody else, so not in L2 yet) and its first K / V tile on the way: a CTA otherwise
       // spends ~2.5 us before its first product can start.  Issued behind this CTA's own
       // first loads (in front of them it delayed them: 1041 instead of 1086 TFLOP/s).
@@ -456,8 +522,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         __syncwarp();
         ++cnt;
       };
-      if (!blk) {
+      if (MODE == kOneItem) {
+        const int n_steps = seq.n;
         // the first product needs Q of tile 0 and the first K tile: those two first, then Q of tile 1
+        load_q(0);
         if (n_steps > 0) load_stage(&tmap_k, seq_start + seq.kv(0) * BN, 0, false);
         load_q(1);
         for (int j = 0; j < n_steps; ++j) {     // K of a step one V earlier when its product is issued ahead
@@ -467,7 +535,53 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           load_stage(&tmap_v, row, 0, false);
           if (j == 1 || n_steps == 1) prefetch_next_cta();   // behind this CTA's own first loads
         }
+      } else if (MANY) {
+        int bid = blockIdx.x, handed = 0;
+        for (int n_ask = 0;; ++n_ask) {
+          int b_, h_, pair_;
+          const bool here = locate(bid, b_, h_, pair_) && place(b_, h_, pair_);
+          if (here) {
+            // the other roles have all taken the item before
+            if (handed > 0) mbar_wait(item_empty, (handed - 1) & 1, abort_flag);
+            if (lane == 0) {
+              item->q0 = q0; item->h = h; item->b = b; item->seq_start = seq_start; item->len = len; item->valid = 1;
+              mbar_arrive(item_full);
+            }
+            __syncwarp();
+            ++handed;
+          }
+          const int n_steps = here ? seq.n : 0;
+          auto ask = [&]() {        // what comes after this item
+            if (elect_one()) {
+              mbar_expect_tx(next_full, 16);
+              try_cancel_next_cta(smem_base + L::kNext, next_full);
+            }
+            __syncwarp();
+          };
+          if (here) load_q(0);       // (in the order the first products need them)
+          if (n_steps > 0) load_stage(&tmap_k, seq_start + seq.kv(0) * BN, 0, false);
+          if (here) load_q(1);
+          if (n_steps < 2) ask();
+          for (int j = 0; j < n_steps; ++j) {
+            const int row = seq_start + seq.kv(j) * BN;
+            if (kAhead && j + 1 < n_steps) load_stage(&tmap_k, seq_start + seq.kv(j + 1) * BN, 0, false);
+            if (!kAhead && j > 0) load_stage(&tmap_k, row, 0, false);
+            load_stage(&tmap_v, row, 0, false);
+            if (j == n_steps - 2) ask();
+          }
+          // (the answer writes shared memory, so it is waited for whatever happened)
+          if (!mbar_wait(next_full, n_ask & 1, abort_flag)) mbar_drain(next_full, n_ask & 1);
+          int y, z;
+          if (__any_sync(0xffffffffu, *abort_flag != 0) || !next_cta(smem_base + L::kNext, bid, y, z)) break;
+          __syncwarp();
+          fence_proxy_async();      // the answer has been read: the next request may overwrite it
+        }
+        if (handed > 0) mbar_wait(item_empty, (handed - 1) & 1, abort_flag);
+        if (lane == 0) { item->valid = 0; mbar_arrive(item_full); }
+        __syncwarp();
       } else {
+        const int n_steps = max(ns0, ns1);
+        load_q(0);
         load_q(1);
         // per tile its own stream, in the order the MMA warp consumes the stages:
         // K(0,0) K(1,0), then per step V(0,j) K(0,j+1) V(1,j) K(1,j+1), or each K before its V
@@ -502,7 +616,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     {
       const uint32_t issue = elect_one() ? 1u : 0u;
       int cnt = 0;
-      int pv_cnt[2] = {0, 0}, qk_cnt[2] = {0, 0};
+      // products issued so far: over all items (barrier phases), and in this item
+      int pv_all[2] = {0, 0}, qk_all[2] = {0, 0}, q_all[2] = {0, 0};
+      int pv_cnt[2] = {0, 0};
       bool q_ready[2] = {false, false};
       // descriptors of stage 0 / tile 0; other stages and k-steps add to the address field
       const uint64_t dq0 = smem_desc_sw128(sQ, 16, 1024);
@@ -516,10 +632,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         return s;
       };
       auto issue_qk = [&](int t, int s) {
-        if (!q_ready[t]) { mbar_wait(q_full(t), 0, abort_flag); tc_fence_after(); q_ready[t] = true; }
+        if (!q_ready[t]) { mbar_wait(q_full(t), MANY ? q_all[t] & 1 : 0, abort_flag); tc_fence_after(); q_ready[t] = true; }
         if (kAhead) {     // the previous scores must be in registers
-          if (qk_cnt[t] > 0) { mbar_wait(s_free(t), (qk_cnt[t] - 1) & 1, abort_flag); tc_fence_after(); }
-          ++qk_cnt[t];
+          if (qk_all[t] > 0) { mbar_wait(s_free(t), (qk_all[t] - 1) & 1, abort_flag); tc_fence_after(); }
+          ++qk_all[t];
         }
         const uint64_t da = dq0 + (uint64_t)((t * L::kQBytes) >> 4);
         const uint64_t db = dk0 + (uint64_t)((s * L::kStageBytes) >> 4);
@@ -531,13 +647,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         mma_commit(s_full(t), issue);
       };
       auto issue_pv = [&](int t, int s) {
-        mbar_wait(p_full(t), pv_cnt[t] & 1, abort_flag);
+        mbar_wait(p_full(t), (MANY ? pv_all[t] : pv_cnt[t]) & 1, abort_flag);
         tc_fence_after();
         const uint64_t db = dv0 + (uint64_t)((s * L::kStageBytes) >> 4);
         mma_ts_x8(tO(t), tP(t), (uint32_t)db, (uint32_t)(db >> 32), kIdescPV, pv_cnt[t] > 0 ? 1u : 0u, issue);
         mma_commit(o_full(t), issue);
         ++pv_cnt[t];
+        if (MANY) ++pv_all[t];
       };
+      for (int n_item = 0; next_item(n_item, [](bool got) { return __all_sync(0xffffffffu, got) != 0; }); ++n_item) {
+      const int n_steps = blk ? max(ns0, ns1) : seq.n;
+      pv_cnt[0] = pv_cnt[1] = 0;
+      q_ready[0] = q_ready[1] = false;
       if (!blk) {
         // both tiles share every K/V stage
         int sK = n_steps > 0 ? wait_stage() : 0;
@@ -596,6 +717,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           }
         }
       }
+      // the item's products have read Q (every phase of q_full is waited for, also where no key was visible)
+      for (int t = 0; t < 2; ++t) {
+        if (!MANY || q0 + kTileM * t >= len) continue;
+        if (!q_ready[t]) mbar_wait(q_full(t), q_all[t] & 1, abort_flag);
+        ++q_all[t];
+        mma_commit(q_free(t), issue);
+      }
+      }
     }
     }
   } else {
@@ -604,17 +733,21 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const int t = warp >> 2;                       // query tile of this warpgroup
     const int row = threadIdx.x & (kTileM - 1);    // row inside the tile == TMEM lane
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const float c = p.scale_log2;
+    int before = 0;           // steps of this tile in the items before (barrier phases)
+    int outs = 0;             // whole output tiles of the items so far, of both tiles
+    for (int n_item = 0; next_item(n_item, [&](bool got) { return !group_any(1 + t, !got); }); ++n_item) {
+    const int n_steps = blk ? max(ns0, ns1) : seq.n;
     const int q0t = q0 + kTileM * t;
     const int qi = q0t + row;                      // query index inside the sequence
-    const float c = p.scale_log2;
     float m_run = -INFINITY;  // max the stored P / O are relative to (raw score units)
     float l_run = 0.f;
-    int items = 0;
+    int items = 0;            // steps of this item
     if (q0t < len) {
       for (int j = 0; j < n_steps; ++j) {
         const int kvt = blk ? 0 : seq.kv(j);
         if (!step_active(t, j)) continue;
-        mbar_wait(s_full(t), items & 1, abort_flag);
+        mbar_wait(s_full(t), (before + items) & 1, abort_flag);
         tc_fence_after();
         uint32_t sr[BN];
 #pragma unroll
@@ -687,7 +820,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const float alpha = (m_use == m_run) ? 1.f : ex2((m_run - m_use) * c);
         const bool rescale = items > 0 && __any_sync(0xffffffffu, alpha != 1.f);
         auto products_done = [&]() {      // O_t holds every product issued so far (and P has been read)
-          mbar_wait(o_full(t), (items - 1) & 1, abort_flag);
+          mbar_wait(o_full(t), (before + items - 1) & 1, abort_flag);
           tc_fence_after();
         };
         auto rescale_o = [&]() {
@@ -758,11 +891,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const long long tok = (long long)seq_start + qi;
       T* orow = (T*)p.o + (p.cu_seqlens ? 0 : (long long)b * p.o_sb) + tok * p.o_st + (long long)h * p.o_sh;
-      uint8_t* sOut = smem_gen + t * L::kQBytes;       // every Q K^T product of this tile has completed
+      // (one item: every Q K^T product of this tile has completed; many: a buffer of its own, shared by
+      // the tiles in turn, so that the next item's Q can be on its way meanwhile)
+      const uint32_t out_off = MANY ? L::kOut : t * L::kQBytes;
+      uint8_t* sOut = smem_gen + out_off;
       if (items > 0) {
-        mbar_wait(o_full(t), (items - 1) & 1, abort_flag);
+        mbar_wait(o_full(t), (before + items - 1) & 1, abort_flag);
         tc_fence_after();
       }
+      const int out_no = outs + ((t == 1 && q0 + kTileM <= len) ? 1 : 0);
+      if (MANY && whole && out_no > 0) mbar_wait(out_free, (out_no - 1) & 1, abort_flag);
 #pragma unroll
       for (int cc = 0; cc < DP / 32; ++cc) {
         uint32_t orr[32];
@@ -794,9 +932,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         else asm volatile("bar.sync 2, 128;" ::: "memory");
         if (row == 0) {
           for (int pn = 0; pn < kPanels; ++pn)
-            tma_store_4d(&tmap_o, sQ + t * L::kQBytes + pn * L::kQPanel, 64 * pn, seq_start + q0t, h, bcoord);
+            tma_store_4d(&tmap_o, smem_base + out_off + pn * L::kQPanel, 64 * pn, seq_start + q0t, h, bcoord);
           bulk_commit_group();
           bulk_wait_read_all();
+          if (MANY) mbar_arrive(out_free);
         }
       }
       if (row_ok && p.lse) {
@@ -804,6 +943,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         if (!p.lse_base2) l2 *= 0.6931471805599453f;
         p.lse[(p.cu_seqlens ? 0 : (long long)b * p.lse_sb) + tok * p.lse_st + (long long)h * p.lse_sh] = l2;
       }
+    }
+    // the next item's first product may overwrite O: this tile's P that lets it start comes later
+    tc_fence_before();
+    if (!MANY) break;
+    before += items;
+    outs += (q0 + kTileM <= len ? 1 : 0) + (q0 + kPairM <= len ? 1 : 0);
     }
   }
 
@@ -891,17 +1036,33 @@ static int validate_prefill(const b200attn_prefill_args* a, bool sparse) {
 }
 
 template <typename T, int DP>
-static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p, cudaStream_t stream) {
+static int launch_prefill(const b200attn_prefill_args* a, PrefillParams& p, cudaStream_t stream) {
   constexpr int BN = 128;
   constexpr int NSTAGE = DP == 128 ? 4 : 6;
-  using L = PrefillSmem<DP, BN, NSTAGE>;
   const long long tokens = a->cu_seqlens ? a->total_tokens : a->seqlen;
   const int tb = a->cu_seqlens ? 1 : a->batch;
-  auto kern = p.block_idx ? prefill_kernel<T, DP, BN, NSTAGE, true> : prefill_kernel<T, DP, BN, NSTAGE, false>;
+  const long long blocks = a->heads_q * (p.packed.seqs > 0 ? packed_tiles_bound(a->batch, a->total_tokens, kPairM, p.n_pairs)
+                                                           : (long long)p.pair_count * a->batch);
+  if (blocks <= 0) return B200ATTN_OK;
+  if (blocks > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
+  // More CTAs than fit at once, and short or ragged walks: CTAs that take over the next item hide its
+  // set-up (place, first loads, ~3000 cycles against 3500 per step) under the end of the one before.
+  // Packed launches, which also look their place up: 12 sequences of 37-3000 tokens 336 -> 329 us (310
+  // -> 296 replayed), 20 of 50-400 59.5 -> 55.3, 64-wide heads 211 -> 197; window 183 -> 172.  Launches
+  // that fit the chip at once are faster one item a CTA (8 heads x 1000 tokens: 19.1 against 20.8 us),
+  // and so are equal lengths (8 x 16 heads x 1024: 59.8 against 60.4; 4 x 32 x 4096, not causal: 1001
+  // against 1007, causal the same), whose CTAs know their place.
+  const bool many = !p.block_idx && blocks > p.prefetch_ahead && (p.packed.seqs > 0 || p.window);
+  const int mode = p.block_idx ? kBlockList : (many ? kManyItems : kOneItem);
+  auto kern = mode == kBlockList ? prefill_kernel<T, DP, BN, NSTAGE, kBlockList>
+              : many             ? prefill_kernel<T, DP, BN, NSTAGE, kManyItems>
+                                 : prefill_kernel<T, DP, BN, NSTAGE, kOneItem>;
+  const int smem = mode == kBlockList ? PrefillSmem<DP, BN, NSTAGE, kBlockList>::kAlloc
+                   : many             ? PrefillSmem<DP, BN, NSTAGE, kManyItems>::kAlloc
+                                      : PrefillSmem<DP, BN, NSTAGE, kOneItem>::kAlloc;
   // the register count is a property of the binary: checked once per instantiation and mode
-  static std::once_flag regs_once[2];
-  static int regs_status[2];
-  const int mode = p.block_idx ? 1 : 0;
+  static std::once_flag regs_once[3];
+  static int regs_status[3];
   std::call_once(regs_once[mode], [kern, mode] {
     cudaFuncAttributes fa;
     regs_status[mode] = (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs >= kLaunchRegs)
@@ -912,7 +1073,7 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
   // the shared-memory opt-in is per device: set on every call (a process may drive several GPUs).
   // Before the tensor maps: it makes the device's context current on this thread, which their encoder
   // needs -- an autograd thread whose allocations all came from a cache may have made no CUDA call yet.
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc) != cudaSuccess)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200ATTN_ERR_CUDA;
   CUtensorMap tq, tk, tv, to;
   if (!make_tmap(&tq, a->dtype, a->q, a->head_dim, tokens, a->heads_q, tb, a->q_stride_t, a->q_stride_h, a->q_stride_b, kTileM) ||
@@ -920,11 +1081,7 @@ static int launch_prefill(const b200attn_prefill_args* a, const PrefillParams& p
       !make_tmap(&tv, a->dtype, a->v, a->head_dim, tokens, a->heads_kv, tb, a->v_stride_t, a->v_stride_h, a->v_stride_b, p.block_idx ? kBlk : BN) ||
       !make_tmap(&to, a->dtype, a->o, a->head_dim, tokens, a->heads_q, tb, a->o_stride_t, a->o_stride_h, a->o_stride_b, kTileM))
     return B200ATTN_ERR_CUDA;
-  const long long blocks = a->heads_q * (p.packed.seqs > 0 ? packed_tiles_bound(a->batch, a->total_tokens, kPairM, p.n_pairs)
-                                                           : (long long)p.pair_count * a->batch);
-  if (blocks <= 0) return B200ATTN_OK;
-  if (blocks > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
-  if (launch_after(kern, dim3((unsigned)blocks), dim3(kPrefillThreads), L::kAlloc, stream, tq, tk, tv, to, p) != cudaSuccess)
+  if (launch_after(kern, dim3((unsigned)blocks), dim3(kPrefillThreads), smem, stream, tq, tk, tv, to, p) != cudaSuccess)
     return B200ATTN_ERR_CUDA;
   set_launch_count(1);
   return cudaGetLastError() == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
@@ -950,7 +1107,8 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
   // a row range ends on a 256-row boundary unless it runs to the end of the longest sequence
   if (!all_rows && row_end < maxlen && row_end % kPairM != 0) return B200ATTN_ERR_SHAPE;
   p.packed = PackedGrid{0, 0};
-  if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch)
+  // (block lists: a CTA finds its own place, ~1 us on its way, and the longest length is known there)
+  if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch && !(sparse && a->sparsity == B200ATTN_BLOCK_LIST))
     p.packed = packed_grid(a->batch, a->total_tokens, (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
   p.pair_begin = row_begin / kPairM;
   p.pair_count = (int)std::min<long long>(p.n_pairs, ((long long)row_end + kPairM - 1) / kPairM) - p.pair_begin;
