@@ -198,30 +198,27 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
   auto pair_of = [&](int it, int& i, int& hq) { i = i_first + it / p.group; hq = hk * p.group + it % p.group; };
   if (warp == kBwdLoadWarp) {
     // ============================================ loader warp: every load, and the dQ reduce-adds
-    BwdCta nx;     // the CTA that will start when one of the resident ones ends
-    const bool have_nx = p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x &&
-                         bwd_cta_of(p, blockIdx.x + p.prefetch_ahead, nx);
+    int n_q[2] = {0, 0}, n_do[2] = {0, 0};     // loads sent into each buffer so far
+    auto load_do = [&](int it) {
+      int i, hq;
+      pair_of(it, i, hq);
+      ++n_do[it & 1];
+      const uint32_t dst = sbase + ((it & 1) ? L::kDO1 : L::kDO), bar = bar_do0 + 8 * (it & 1);
+      mbar_expect_tx(bar, L::kOperand);
+      for (int pn = 0; pn < kPanels; ++pn)
+        tma_load_4d(dst + pn * L::kPanel, &tmap_do, bar, 64 * pn, seq_start + i * kT, hq, bcoord);
+    };
+    auto load_q = [&](int it) {
+      int i, hq;
+      pair_of(it, i, hq);
+      ++n_q[it & 1];
+      const uint32_t dst = sbase + ((it & 1) ? L::kQ1 : L::kQ), bar = bar_q0 + 8 * (it & 1);
+      mbar_expect_tx(bar, L::kOperand);
+      for (int pn = 0; pn < kPanels; ++pn)
+        tma_load_4d(dst + pn * L::kPanel, &tmap_q, bar, 64 * pn, seq_start + i * kT, hq, bcoord);
+    };
     if (elect_one()) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_do);
-      int n_q[2] = {0, 0}, n_do[2] = {0, 0};     // loads sent into each buffer so far
-      auto load_do = [&](int it) {
-        int i, hq;
-        pair_of(it, i, hq);
-        ++n_do[it & 1];
-        const uint32_t dst = sbase + ((it & 1) ? L::kDO1 : L::kDO), bar = bar_do0 + 8 * (it & 1);
-        mbar_expect_tx(bar, L::kOperand);
-        for (int pn = 0; pn < kPanels; ++pn)
-          tma_load_4d(dst + pn * L::kPanel, &tmap_do, bar, 64 * pn, seq_start + i * kT, hq, bcoord);
-      };
-      auto load_q = [&](int it) {
-        int i, hq;
-        pair_of(it, i, hq);
-        ++n_q[it & 1];
-        const uint32_t dst = sbase + ((it & 1) ? L::kQ1 : L::kQ), bar = bar_q0 + 8 * (it & 1);
-        mbar_expect_tx(bar, L::kOperand);
-        for (int pn = 0; pn < kPanels; ++pn)
-          tma_load_4d(dst + pn * L::kPanel, &tmap_q, bar, 64 * pn, seq_start + i * kT, hq, bcoord);
-      };
       // in the order the first products need them: K and Q(0) for S^T, V and dO(0) for dP^T
       mbar_expect_tx(bar_kv, 2 * L::kOperand);
       for (int pn = 0; pn < kPanels; ++pn)
@@ -231,6 +228,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
         tma_load_4d(sbase + L::kV + pn * L::kPanel, &tmap_v, bar_kv, 64 * pn, seq_start + kv0, hk, bcoord);
       load_do(0);
       if (n_iter > 1) { load_q(1); load_do(1); }
+    }
+    __syncwarp();
+    // (behind the first loads: a packed launch looks that CTA up in the lengths, ~1 us)
+    BwdCta nx;     // the CTA that will start when one of the resident ones ends
+    const bool have_nx = p.prefetch_ahead > 0 && blockIdx.x + p.prefetch_ahead < gridDim.x &&
+                         bwd_cta_of(p, blockIdx.x + p.prefetch_ahead, nx);
+    if (elect_one()) {
       // That next CTA finds its K / V tile and its first Q / dO tiles on their way into L2.
       if (have_nx) {
         int ss2 = 0, len2 = p.seqlen, bc2 = nx.b;

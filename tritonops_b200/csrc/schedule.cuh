@@ -54,18 +54,30 @@ inline long long packed_tiles_bound(int batch, long long total_tokens, int tile,
 __device__ __forceinline__ bool packed_item(const PackedGrid g, const int32_t* __restrict__ cu, int batch, int tile,
                                             int max_tiles, int heads, int idx, PackedItem& out) {
   const int lane = threadIdx.x & 31;
+  auto tiles_of = [&](int c) {   // of this lane's sequence in chunk c
+    const int b = c * g.seqs + lane;
+    if (lane >= g.seqs || b >= batch) return 0;
+    const int len = cu[b + 1] - cu[b];
+    return len > 0 ? min((len - 1) / tile + 1, max_tiles) : 0;
+  };
   int np = 0, b0 = 0, total = 0;
   bool found = false;
-  for (int c = 0; c < g.n_chunks; ++c) {
-    const int b = c * g.seqs + lane;
-    int n = 0;
-    if (lane < g.seqs && b < batch) {
-      const int len = cu[b + 1] - cu[b];
-      n = len > 0 ? min((len - 1) / tile + 1, max_tiles) : 0;
+  if (g.n_chunks == 1) {
+    np = tiles_of(0);
+    total = __reduce_add_sync(0xffffffffu, np);
+    found = idx < total * heads;
+  } else {
+    int n[kSchedMaxChunks];      // (all loads in flight at once)
+#pragma unroll
+    for (int c = 0; c < kSchedMaxChunks; ++c) n[c] = c < g.n_chunks ? tiles_of(c) : 0;
+#pragma unroll
+    for (int c = 0; c < kSchedMaxChunks; ++c) {
+      if (!found && c < g.n_chunks) {
+        const int sum = __reduce_add_sync(0xffffffffu, n[c]);
+        if (idx < sum * heads) { np = n[c]; b0 = c * g.seqs; total = sum; found = true; }
+        else idx -= sum * heads;
+      }
     }
-    const int sum = __reduce_add_sync(0xffffffffu, n);
-    if (idx < sum * heads) { np = n; b0 = c * g.seqs; total = sum; found = true; break; }
-    idx -= sum * heads;
   }
   if (!found) return false;
   const int per_group = total * kSchedHeads;
@@ -74,6 +86,12 @@ __device__ __forceinline__ bool packed_item(const PackedGrid g, const int32_t* _
   const int g_heads = min(kSchedHeads, heads - grp * kSchedHeads);
   const int rank = in_grp / g_heads;               // heaviest first, over the sequences of the chunk
   out.head = grp * kSchedHeads + in_grp - rank * g_heads;
+  if (g.seqs == 1) {                               // one sequence: its tiles from the heaviest down
+    out.level = total - 1 - rank;
+    out.b = b0;
+    out.n_tiles = total;
+    return true;
+  }
   // the level of that rank: the largest L with more than `rank` tiles at levels >= L
   int lo = 0, hi = __reduce_max_sync(0xffffffffu, np);      // C(lo) > rank, C(hi) = 0
   int above = 0;                                             // C(hi)
