@@ -207,9 +207,11 @@ struct PrefillItem {
   int valid;              // 0: no more items
 };
 
-// What a CTA works on: one item found from its coordinates, items handed out until none is left, or
-// one item with block-list sparsity (own instantiations, so that none carries the others' branches).
-enum PrefillMode { kOneItem, kManyItems, kBlockList };
+// What a CTA works on: one item found from its coordinates, one item of a packed launch, items handed
+// out until none is left, or one item with block-list sparsity.  Own instantiations, so that none
+// carries the others' code: the packed look-up alone, never run, cost the dense kernel 2 % (4 x 32 heads
+// x 4096, replayed: 518 against 505 us).
+enum PrefillMode { kOneItem, kOnePacked, kManyItems, kBlockList };
 
 template <int DP, int BN, int NSTAGE, PrefillMode MODE>
 struct PrefillSmem {
@@ -319,7 +321,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   const int n_bh = p.batch * p.heads_q;
   const int per_group = kHeadGroup * p.pair_count;
   auto locate = [&](int bid, int& b_, int& h_, int& pair_) -> bool {
-    if (p.packed.seqs > 0) {
+    if (MODE == kOnePacked || (MANY && p.packed.seqs > 0)) {
       PackedItem it;
       if (!packed_item(p.packed, p.cu_seqlens, p.batch, kPairM, p.n_pairs, p.heads_q, bid, it)) return false;
       b_ = it.b; h_ = it.head; pair_ = it.level;
@@ -522,7 +524,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         __syncwarp();
         ++cnt;
       };
-      if (MODE == kOneItem) {
+      if (MODE == kOneItem || MODE == kOnePacked) {
         const int n_steps = seq.n;
         // the first product needs Q of tile 0 and the first K tile: those two first, then Q of tile 1
         load_q(0);
@@ -1053,16 +1055,18 @@ static int launch_prefill(const b200attn_prefill_args* a, PrefillParams& p, cuda
   // and so are equal lengths (8 x 16 heads x 1024: 59.8 against 60.4; 4 x 32 x 4096, not causal: 1001
   // against 1007, causal the same), whose CTAs know their place.
   const bool many = !p.block_idx && blocks > p.prefetch_ahead && (p.packed.seqs > 0 || p.window);
-  const int mode = p.block_idx ? kBlockList : (many ? kManyItems : kOneItem);
-  auto kern = mode == kBlockList ? prefill_kernel<T, DP, BN, NSTAGE, kBlockList>
-              : many             ? prefill_kernel<T, DP, BN, NSTAGE, kManyItems>
-                                 : prefill_kernel<T, DP, BN, NSTAGE, kOneItem>;
-  const int smem = mode == kBlockList ? PrefillSmem<DP, BN, NSTAGE, kBlockList>::kAlloc
-                   : many             ? PrefillSmem<DP, BN, NSTAGE, kManyItems>::kAlloc
-                                      : PrefillSmem<DP, BN, NSTAGE, kOneItem>::kAlloc;
+  const PrefillMode mode = p.block_idx ? kBlockList : many ? kManyItems : p.packed.seqs > 0 ? kOnePacked : kOneItem;
+  void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams) = nullptr;
+  int smem = 0;
+  switch (mode) {
+    case kBlockList: kern = prefill_kernel<T, DP, BN, NSTAGE, kBlockList>; smem = PrefillSmem<DP, BN, NSTAGE, kBlockList>::kAlloc; break;
+    case kManyItems: kern = prefill_kernel<T, DP, BN, NSTAGE, kManyItems>; smem = PrefillSmem<DP, BN, NSTAGE, kManyItems>::kAlloc; break;
+    case kOnePacked: kern = prefill_kernel<T, DP, BN, NSTAGE, kOnePacked>; smem = PrefillSmem<DP, BN, NSTAGE, kOnePacked>::kAlloc; break;
+    default: kern = prefill_kernel<T, DP, BN, NSTAGE, kOneItem>; smem = PrefillSmem<DP, BN, NSTAGE, kOneItem>::kAlloc; break;
+  }
   // the register count is a property of the binary: checked once per instantiation and mode
-  static std::once_flag regs_once[3];
-  static int regs_status[3];
+  static std::once_flag regs_once[4];
+  static int regs_status[4];
   std::call_once(regs_once[mode], [kern, mode] {
     cudaFuncAttributes fa;
     regs_status[mode] = (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs >= kLaunchRegs)
