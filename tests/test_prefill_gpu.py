@@ -162,6 +162,28 @@ def test_window_prefill(dtype, L, G):
     assert bool((lse2.cpu()[~fin] == -math.inf).all())
 
 
+# one item per CTA, and 432 items for CTAs that take them over; both head widths of the kernel
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("lens,h,d", [([200, 1, 128], 2, 128), ([200, 1, 128], 2, 64), ([300, 700, 129] * 6, 12, 128),
+                                      ([300, 700, 129] * 6, 12, 64)])
+def test_rows_without_a_visible_key_are_zero(dtype, lens, h, d):
+    """An empty window, and block lists that name nothing a row may see: O = 0 and LSE = -inf."""
+    ops, _, _, _ = _mods()
+    q, k, v, cu = (t.cuda() for t in make(lens, h, h, d, dtype, seed=3))
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu, sparsity=ops.WINDOW, window_local=0, window_global=0)
+    assert o.abs().max() == 0 and bool((lse == -math.inf).all())
+    nb = (max(lens) + 63) // 64
+    idx = torch.full((len(lens), h, nb, 2), nb - 1, dtype=torch.int32, device="cuda")   # the last block only
+    cnt = torch.ones(len(lens), h, nb, dtype=torch.int32, device="cuda")
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu, max_seqlen=max(lens), sparsity=ops.BLOCK_LIST, block_idx=idx,
+                         block_cnt=cnt)
+    at = cu.tolist()
+    for b, n in enumerate(lens):
+        seen = n if (n + 63) // 64 < nb else (nb - 1) * 64      # rows before the listed block, or none of it there
+        s = slice(at[b], at[b] + seen)
+        assert o[:, s].abs().max() == 0 and bool((lse[:, s] == -math.inf).all())
+
+
 def test_cfg2_shape_properties():
     """Full config 2 (B=4,H=32,S=4096,D=128 causal bf16): sampled heads against
     fp32 math on the device, determinism, and prefix invariance (causal rows do

@@ -156,9 +156,10 @@ __device__ __forceinline__ void ffma2v(float& d0, float& d1, float a0, float a1,
 // per SM and is as busy as the tensor core in this kernel): x = n + f with n = round(x),
 // 2^f by a cubic on [-0.5, 0.5] (relative error 1e-4, below the 16-bit P it feeds), n added
 // into the exponent field.  x <= ~9 here; x below -125, masked scores (-inf) included, gives
-// 2^-125 = 2.4e-38 rather than 0: every row that reaches this code has a visible key whose
-// term is at least 2^-8, so the difference is below 1e-35 relative (guarding it with a
-// compare + select per value cost more than the cubic saved: 1034 instead of 1070 TFLOP/s).
+// 2^-125 = 2.4e-38 rather than 0: beside a visible key, whose term is at least 2^-8, that is
+// below 1e-35 relative (guarding it with a compare + select per value cost more than the cubic
+// saved: 1034 instead of 1070 TFLOP/s).  A row without any visible key has nothing else in its
+// sums; the epilogue tells it by its maximum, which is still -inf.
 __device__ __forceinline__ void exp2_fma_pair(float& e0, float& e1, float x0, float x1) {
   const float magic = 12582912.f;   // 1.5 * 2^23: adding it leaves round(x) in the low mantissa bits
   x0 = fmaxf(x0, -125.f);
@@ -890,7 +891,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // per-thread stores, which leave the next packed sequence's rows alone.
       const bool row_ok = qi < len;
       const bool whole = q0t + kTileM <= len;
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      // (no visible key: O = 0, whatever the masked columns left in the sums)
+      const float inv = (l_run > 0.f && m_run != -INFINITY) ? 1.f / l_run : 0.f;
       const long long tok = (long long)seq_start + qi;
       T* orow = (T*)p.o + (p.cu_seqlens ? 0 : (long long)b * p.o_sb) + tok * p.o_st + (long long)h * p.o_sh;
       // (one item: every Q K^T product of this tile has completed; many: a buffer of its own, shared by
