@@ -34,9 +34,9 @@ __global__ void pack_to_cache_kernel(const uint4* __restrict__ packed, uint4* __
 }
 
 // cache[b, len_b, h, :] = new_rows[b, h, :]   (rows with len_b >= capacity are skipped)
-__global__ void append_kernel(const uint4* __restrict__ new_k, const uint4* __restrict__ new_v,
+__global__ void append_kernel(const uint4* new_k, const uint4* new_v,
                               uint4* __restrict__ k_cache, uint4* __restrict__ v_cache,
-                              const int32_t* __restrict__ seqlens, long long n_sb, long long n_sh,
+                              const int32_t* seqlens, long long n_sb, long long n_sh,
                               long long c_sb, long long c_st, long long c_sh, int batch, int capacity,
                               int heads, int vec_per_row) {
   // (a decoding kernel behind this one is set up meanwhile, as this one is behind the step before)

@@ -594,7 +594,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ C
 // D[t, h] = sum_d dO[t, h, d] * O[t, h, d], and the row's fp32 dQ accumulator cleared (saves a
 // separate memset pass over it): eight lanes per (token, head) with 16-byte loads.
 template <typename T>
-__global__ void bwd_rowsum_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ dvec,
+__global__ void bwd_rowsum_kernel(const T* o, const T* d_o, float* __restrict__ dvec,
                                   float* __restrict__ dq_acc, long long o_sb, long long o_st, long long o_sh,
                                   long long do_sb, long long do_st, long long do_sh, int tokens_per_batch, int heads,
                                   int D, int DP, long long total) {
@@ -628,7 +628,7 @@ __global__ void bwd_rowsum_kernel(const T* __restrict__ o, const T* __restrict__
 
 // dq[t, h, :D] = T(dq_acc[t, h, :D])
 template <typename T>
-__global__ void bwd_convert_dq_kernel(const float* __restrict__ acc, T* __restrict__ dq, long long dq_sb,
+__global__ void bwd_convert_dq_kernel(const float* acc, T* __restrict__ dq, long long dq_sb,
                                       long long dq_st, long long dq_sh, int tokens_per_batch, int heads, int D,
                                       int DP, long long total_rows) {
   grid_dependency_wait();

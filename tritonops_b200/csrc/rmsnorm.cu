@@ -175,7 +175,7 @@ constexpr int kFwdStreamThreads = 32 * (kFwdStreamConsumers + 1);
 
 template <typename XT, typename WT>
 __global__ void __launch_bounds__(kFwdStreamThreads, 1)
-rmsnorm_fwd_stream_kernel(const XT* __restrict__ x, const WT* __restrict__ w, XT* __restrict__ y,
+rmsnorm_fwd_stream_kernel(const XT* x, const WT* w, XT* __restrict__ y,
                           float* __restrict__ rstd, long long rows, int D, long long xs, long long ys, float eps,
                           int slot_bytes, int n_slots) {
   using namespace sm100;
@@ -294,8 +294,8 @@ constexpr int kBwdStreamThreads = 32 * (kBwdStreamConsumers + 1);
 
 template <typename XT, typename WT, int CH>
 __global__ void __launch_bounds__(kBwdStreamThreads, 1)
-rmsnorm_bwd_stream_kernel(const XT* __restrict__ dy, const XT* __restrict__ x, const WT* __restrict__ w,
-                          const float* __restrict__ rstd, XT* __restrict__ dx, float* __restrict__ partial,
+rmsnorm_bwd_stream_kernel(const XT* dy, const XT* x, const WT* w, const float* rstd,
+                          XT* __restrict__ dx, float* __restrict__ partial,
                           long long rows, int D, long long dys, long long xs, long long dxs, int slot_bytes,
                           int n_slots) {
   using namespace sm100;
@@ -602,7 +602,7 @@ rmsnorm_bwd_vec_kernel(const XT* __restrict__ dy, const XT* __restrict__ x, cons
 constexpr int kDwRows = 32;
 template <typename WT>
 __global__ void __launch_bounds__(32 * kDwRows)
-rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, WT* __restrict__ dw, int D, int n_partial) {
+rmsnorm_dw_reduce_kernel(const float* partial, WT* __restrict__ dw, int D, int n_partial) {
   sm100::grid_dependency_wait();
   __shared__ float part[kDwRows][33];
   const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;

@@ -51,7 +51,7 @@ inline long long packed_tiles_bound(int batch, long long total_tokens, int tile,
 }
 
 // Item `idx` of the launch; false when there are fewer.  Executed by whole converged warps.
-__device__ __forceinline__ bool packed_item(const PackedGrid g, const int32_t* __restrict__ cu, int batch, int tile,
+__device__ __forceinline__ bool packed_item(const PackedGrid g, const int32_t* cu, int batch, int tile,
                                             int max_tiles, int heads, int idx, PackedItem& out) {
   const int lane = threadIdx.x & 31;
   auto tiles_of = [&](int c) {   // of this lane's sequence in chunk c

@@ -28,6 +28,8 @@ __device__ __forceinline__ bool elect_one() {
 // A kernel launched with programmatic stream serialisation may begin while the one before it on
 // the stream still runs; what that one wrote is visible after the wait (a no-op when launched the
 // ordinary way).  The other call lets the next kernel on the stream begin, if it was launched so.
+// What is read behind the wait may have changed while this kernel was already running, so it is not
+// read-only data for the kernel: no `const ... __restrict__` parameters and no ld.global.nc there.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
