@@ -9,7 +9,6 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libb200attn.so")
-HOST_PATH = os.path.join(_HERE, "csrc", "_b200host.so")
 
 F16, BF16, F32 = 0, 1, 2
 DENSE, WINDOW, BLOCK_LIST = 0, 1, 2
@@ -155,23 +154,28 @@ SYMBOLS = {
 }
 NOALLOC_SCRATCH_BYTES = 32 << 20
 
+# the argument structs csrc/host.cpp fills, in the order its init() takes their sizes
+HOST_STRUCTS = (PrefillArgs, PrefillBwdArgs, DecodeArgs, PagedDecodeArgs, KvAppendArgs, TopkBlocksArgs, RmsNormFwdArgs,
+                RmsNormBwdArgs)
+
 _lib = None
 _host = None
 
 
 def host():
     """The native call path of ops.py (csrc/host.cpp), bound to the library; raises if it has not
-    been built."""
+    been built for this torch and Python, or with other argument structs than the ones here."""
     global _host
     if _host is None:
-        path = LIB_PATH
+        from .build import host_path
+        path = host_path()
         lib()
-        if not os.path.exists(HOST_PATH):
-            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m tritonops_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_b200host", HOST_PATH)
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m tritonops_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_b200host", path)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200host", loader))
         loader.exec_module(module)
-        module.init(path)
+        module.init(LIB_PATH, *(C.sizeof(s) for s in HOST_STRUCTS))
         _host = module
     return _host
 

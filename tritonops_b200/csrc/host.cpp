@@ -423,9 +423,21 @@ bool bind(void* h, const char* name, F& fn) {
   return fn != nullptr;
 }
 
-// init(path of libb200attn.so): resolve its entry points
-PyObject* init(PyObject*, PyObject* path) {
-  const char* p = PyUnicode_AsUTF8(path);
+// init(path of libb200attn.so, sizes of the argument structs as the caller knows them): resolve its
+// entry points
+PyObject* init(PyObject*, PyObject* const* x, Py_ssize_t n) {
+  const size_t sizes[] = {sizeof(b200attn_prefill_args), sizeof(b200attn_prefill_bwd_args), sizeof(b200attn_decode_args),
+                          sizeof(b200attn_paged_decode_args), sizeof(b200attn_kv_append_args),
+                          sizeof(b200attn_topk_blocks_args), sizeof(b200attn_rmsnorm_fwd_args),
+                          sizeof(b200attn_rmsnorm_bwd_args)};
+  constexpr Py_ssize_t kStructs = sizeof(sizes) / sizeof(sizes[0]);
+  bool same = n == 1 + kStructs;
+  for (Py_ssize_t i = 0; same && i < kStructs; ++i) same = PyLong_AsSize_t(x[1 + i]) == sizes[i];
+  if (!same) {
+    PyErr_Clear();
+    return PyErr_Format(PyExc_RuntimeError, "the native call path was built with other argument structs; rebuild it");
+  }
+  const char* p = PyUnicode_AsUTF8(x[0]);
   if (!p) return nullptr;
   void* h = dlopen(p, RTLD_NOW | RTLD_LOCAL);
   if (!h) return PyErr_Format(PyExc_RuntimeError, "%s", dlerror());
@@ -446,7 +458,7 @@ PyObject* init(PyObject*, PyObject* path) {
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST(prefill), FAST(prefill_bwd), FAST(decode), FAST(paged_decode), FAST(append_kv),
                          FAST(topk_blocks), FAST(rmsnorm_fwd), FAST(rmsnorm_bwd),
-                         {"init", init, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         FAST(init), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
