@@ -1118,10 +1118,11 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
   p.n_pairs = (maxlen + kPairM - 1) / kPairM;
   // a row range ends on a 256-row boundary unless it runs to the end of the longest sequence
   if (!all_rows && row_end < maxlen && row_end % kPairM != 0) return B200ATTN_ERR_SHAPE;
-  p.packed = PackedGrid{0, 0};
+  p.packed = PackedGrid{};
   // (block lists: a CTA finds its own place, ~1 us on its way, and the longest length is known there)
   if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch && !(sparse && a->sparsity == B200ATTN_BLOCK_LIST))
-    p.packed = packed_grid(a->batch, a->total_tokens, (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
+    p.packed = packed_grid(a->batch, a->total_tokens, a->heads_q, a->causal || (sparse && a->sparsity == B200ATTN_WINDOW),
+                           (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
   p.pair_begin = row_begin / kPairM;
   p.pair_count = (int)std::min<long long>(p.n_pairs, ((long long)row_end + kPairM - 1) / kPairM) - p.pair_begin;
   if (p.pair_count <= 0) return B200ATTN_OK;

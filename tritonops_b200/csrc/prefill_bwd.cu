@@ -813,10 +813,11 @@ int prefill_bwd(const b200attn_prefill_bwd_args* a, cudaStream_t stream) {
   const int maxlen = a->cu_seqlens ? a->max_seqlen : a->seqlen;
   p.n_kvtiles = (maxlen + kT - 1) / kT;
   if (p.n_kvtiles <= 0) return B200ATTN_OK;
-  p.packed = PackedGrid{0, 0};
+  p.packed = PackedGrid{};
   if (a->cu_seqlens && a->batch <= kSchedMaxBatch)
     // what should stay in L2 here is the fp32 dQ accumulator of the head group (and its Q, dO)
-    p.packed = packed_grid(a->batch, a->total_tokens, (long long)kSchedHeads * p.group * dpad(a->head_dim) * 8);
+    p.packed = packed_grid(a->batch, a->total_tokens, a->heads_kv, a->causal,
+                           (long long)kSchedHeads * p.group * dpad(a->head_dim) * 8);
   p.causal = a->causal ? 1 : 0;
   p.scale = a->softmax_scale * (a->scale_has_log2e ? 0.6931471805599453f : 1.f);
   p.scale_log2 = a->softmax_scale * (a->scale_has_log2e ? 1.f : 1.4426950408889634f);
