@@ -607,9 +607,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           }
         }
       }
-      // every issued copy must have landed before the CTA may exit (Q too: a tile with an empty list, or
-      // after a wait gave up, is not waited for by the products)
-      for (int t = 0; t < 2; ++t)
+      // every issued copy must have landed before the CTA may exit (Q too: a tile with an empty list is not
+      // waited for by the products, nor any after a wait gave up)
+      for (int t = 0; t < 2 && (BLK || *abort_flag != 0); ++t)
         if (q_loads[t] > 0 && !mbar_wait(q_full(t), (q_loads[t] - 1) & 1, abort_flag))
           mbar_drain(q_full(t), (q_loads[t] - 1) & 1);
       for (int c = max(cnt - NSTAGE, 0); c < cnt; ++c)
@@ -906,7 +906,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       if (items > 0) {
         mbar_wait(o_full(t), (before + items - 1) & 1, abort_flag);
         tc_fence_after();
-      } else if (!MANY) {
+      } else if (BLK) {       // (in the other modes every tile has a step)
         mbar_wait(q_full(t), 0, abort_flag);     // no product has waited for Q: it may still be on its way
       }
       const int out_no = outs + ((t == 1 && q0 + kTileM <= len) ? 1 : 0);
