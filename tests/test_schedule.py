@@ -37,20 +37,23 @@ static int __popc(unsigned v) { return __builtin_popcount(v); }
 static int __ffs(unsigned v) { return __builtin_ffs((int)v); }
 #include "schedule.cuh"
 using namespace b200attn;
-// argv: tile max_tiles heads causal kv_bytes len...; prints the grid, then "b head level n_tiles" per item
+// argv: tile max_tiles heads causal kv_bytes equal len...; prints the grid, then "b head level n_tiles" per item
 int main(int argc, char** argv) {
   auto num = [&](int i) { return atoll(argv[i]); };
-  const int tile = num(1), max_tiles = num(2), heads = num(3), batch = argc - 6;
+  const int tile = num(1), max_tiles = num(2), heads = num(3), batch = argc - 7;
   std::vector<int32_t> cu(1, 0);
-  for (int i = 6; i < argc; ++i) cu.push_back(cu.back() + (int)num(i));
-  const PackedGrid g = packed_grid(batch, cu.back(), heads, num(4) != 0, num(5));
+  for (int i = 7; i < argc; ++i) cu.push_back(cu.back() + (int)num(i));
+  PackedGrid g = packed_grid(batch, cu.back(), heads, num(4) != 0, num(5));
+  if (num(6) && equal_lengths(batch, cu.back(), (int)num(7))) g.equal = ((int)num(7) + tile - 1) / tile;
   const int items = (int)packed_tiles_bound(batch, cu.back(), tile, max_tiles) * heads;
-  printf("%d %d %d\n", g.seqs, g.n_chunks, g.heads);
+  printf("%d %d %d %d %d\n", g.seqs, g.n_chunks, g.heads, g.equal, (int)tight_grid(batch, cu.back(), tile, max_tiles));
   auto lane = [&](int l) {
     threadIdx.x = l;
     for (int i = 0; i < items; ++i) {
       PackedItem it = {-1, -1, -1, -1};
-      const bool there = packed_item(g, cu.data(), batch, tile, max_tiles, heads, i, it);
+      bool there = true;
+      if (g.equal > 0) equal_item(g, batch, heads, i, it);
+      else there = packed_item(g, cu.data(), batch, tile, max_tiles, heads, i, it);
       if (l == 0) { if (there) printf("%d %d %d %d\n", it.b, it.head, it.level, it.n_tiles); else printf("-\n"); }
     }
   };
@@ -71,8 +74,8 @@ def run(tmp_path_factory):
     subprocess.check_call(["g++", "-std=c++20", "-O1", "-pthread", "-I", os.path.join(ROOT, "tritonops_b200", "csrc"),
                            "-o", str(exe), str(d / "harness.cpp")])
 
-    def call(lens, heads, causal, tile=256, max_tiles=1 << 20, kv_bytes=2048):
-        args = [tile, max_tiles, heads, int(causal), kv_bytes, *lens]
+    def call(lens, heads, causal, tile=256, max_tiles=1 << 20, kv_bytes=2048, equal=False):
+        args = [tile, max_tiles, heads, int(causal), kv_bytes, int(equal), *lens]
         out = subprocess.run([str(exe), *map(str, args)], capture_output=True, text=True, check=True).stdout.split("\n")
         return [int(x) for x in out[0].split()], [tuple(map(int, x.split())) for x in out[1:] if x and x != "-"]
     return call
@@ -91,7 +94,7 @@ def _batches():
 @pytest.mark.parametrize("kv_bytes", [2048, 1 << 16])       # chunks of many sequences, and of one or a few
 def test_every_tile_once_and_the_heaviest_first(run, causal, kv_bytes):
     for lens, heads, max_tiles in _batches():
-        (seqs, n_chunks, group), items = run(lens, heads, causal, max_tiles=max_tiles, kv_bytes=kv_bytes)
+        (seqs, n_chunks, group, _, _), items = run(lens, heads, causal, max_tiles=max_tiles, kv_bytes=kv_bytes)
         tiles = [min(-(-n // 256), max_tiles) for n in lens]
         assert sorted(i[:3] for i in items) == sorted((b, h, t) for b, n in enumerate(tiles) for h in range(heads)
                                                       for t in range(n))
@@ -110,3 +113,21 @@ def test_every_tile_once_and_the_heaviest_first(run, causal, kv_bytes):
 def test_head_groups_are_of_one_size(run):
     for heads, want in [(1, 1), (8, 8), (9, 5), (12, 6), (16, 8), (28, 7), (40, 8)]:
         assert run([1], heads, True)[0][2] == want
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("batch,n,heads,kv_bytes", [(1, 1500, 9, 2048), (5, 600, 12, 2048), (7, 256, 8, 1 << 17), (40, 257, 1, 2048)])
+def test_equal_lengths_are_handed_out_in_the_same_order(run, causal, batch, n, heads, kv_bytes):
+    grid, items = run([n] * batch, heads, causal, max_tiles=-(-n // 256), kv_bytes=kv_bytes)
+    fast, same = run([n] * batch, heads, causal, max_tiles=-(-n // 256), kv_bytes=kv_bytes, equal=True)
+    assert grid[3] == 0 and fast[3] == -(-n // 256)
+    assert same == items
+    # other lengths of the same sum are not taken for equal ones
+    if batch > 1:
+        assert run([n - 1] + [n] * (batch - 2) + [n + 1], heads, causal, equal=True)[0][3] == 0
+
+
+def test_which_grids_are_tight(run):
+    """Longest 3000: four sequences of that length, of half that length, one among short ones."""
+    for lens, want in [([3000] * 4, 1), ([3000, 1600, 1500, 1400], 1), ([3000, 100, 100, 100], 0)]:
+        assert run(lens, 1, True, max_tiles=12)[0][4] == want

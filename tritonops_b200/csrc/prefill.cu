@@ -324,7 +324,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   auto locate = [&](int bid, int& b_, int& h_, int& pair_) -> bool {
     if (MODE == kOnePacked || (MANY && p.packed.seqs > 0)) {
       PackedItem it;
-      if (!packed_item(p.packed, p.cu_seqlens, p.batch, kPairM, p.n_pairs, p.heads_q, bid, it)) return false;
+      if (p.packed.equal > 0) equal_item(p.packed, p.batch, p.heads_q, bid, it);
+      else if (!packed_item(p.packed, p.cu_seqlens, p.batch, kPairM, p.n_pairs, p.heads_q, bid, it)) return false;
       b_ = it.b; h_ = it.head; pair_ = it.level;
       return true;
     }
@@ -1055,14 +1056,19 @@ static int launch_prefill(const b200attn_prefill_args* a, PrefillParams& p, cuda
                                                            : (long long)p.pair_count * a->batch);
   if (blocks <= 0) return B200ATTN_OK;
   if (blocks > 0x7fffffffLL) return B200ATTN_ERR_TOO_LARGE;
-  // More CTAs than fit at once, and short or ragged walks: CTAs that take over the next item hide its
+  // More than two CTAs per SM, and short or ragged walks: CTAs that take over the next item hide its
   // set-up (place, first loads, ~3000 cycles against 3500 per step) under the end of the one before.
   // Packed launches, which also look their place up: 12 sequences of 37-3000 tokens 336 -> 329 us (310
-  // -> 296 replayed), 20 of 50-400 59.5 -> 55.3, 64-wide heads 211 -> 197; window 183 -> 172.  Launches
-  // that fit the chip at once are faster one item a CTA (8 heads x 1000 tokens: 19.1 against 20.8 us),
-  // and so are equal lengths (8 x 16 heads x 1024: 59.8 against 60.4; 4 x 32 x 4096, not causal: 1001
-  // against 1007, causal the same), whose CTAs know their place.
-  const bool many = !p.block_idx && blocks > p.prefetch_ahead && (p.packed.seqs > 0 || p.window);
+  // -> 296 replayed), 20 of 50-400 59.5 -> 55.3, 64-wide heads 211 -> 197.  Windows: 2 x 6000-9000 tokens,
+  // 16 heads, local 1024 181 -> 177; 2 x 4096, local 64 50.2 -> 46.0, local 2048 115.8 -> 116.0.  With
+  // fewer CTAs the second items end unevenly (windows of 160 CTAs, local 2048: 41.4 one item a CTA, 43.3
+  // so; 256 CTAs 64.0 and 65.2), unless they are brief (160 CTAs, local 64: 24.5 and 24.0; 32 x 128 tokens,
+  // 256 CTAs, 16.5 and 15.5).  Launches that fit the chip at once are faster one item a CTA (8 heads x 1000
+  // tokens: 19.1 against 20.8), and so are calls without cu_seqlens (8 x 16 heads x 1024: 59.8 against 60.4;
+  // 4 x 32 x 4096, not causal: 1001 against 1007, causal the same).
+  const bool brief = p.window ? (long long)p.win_local + p.win_global <= 5 * BN
+                              : a->cu_seqlens && a->total_tokens <= (long long)kPairM * a->batch;
+  const bool many = !p.block_idx && blocks > (brief ? 1LL : 2LL) * p.prefetch_ahead && (p.packed.seqs > 0 || p.window);
   const PrefillMode mode = p.block_idx ? kBlockList : many ? kManyItems : p.packed.seqs > 0 ? kOnePacked : kOneItem;
   void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PrefillParams) = nullptr;
   int smem = 0;
@@ -1118,11 +1124,6 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
   p.n_pairs = (maxlen + kPairM - 1) / kPairM;
   // a row range ends on a 256-row boundary unless it runs to the end of the longest sequence
   if (!all_rows && row_end < maxlen && row_end % kPairM != 0) return B200ATTN_ERR_SHAPE;
-  p.packed = PackedGrid{};
-  // (block lists: a CTA finds its own place, ~1 us on its way, and the longest length is known there)
-  if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch && !(sparse && a->sparsity == B200ATTN_BLOCK_LIST))
-    p.packed = packed_grid(a->batch, a->total_tokens, a->heads_q, a->causal || (sparse && a->sparsity == B200ATTN_WINDOW),
-                           (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
   p.pair_begin = row_begin / kPairM;
   p.pair_count = (int)std::min<long long>(p.n_pairs, ((long long)row_end + kPairM - 1) / kPairM) - p.pair_begin;
   if (p.pair_count <= 0) return B200ATTN_OK;
@@ -1136,6 +1137,24 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
     p.prefetch_ahead = di->sm_count * B200ATTN_PREFETCH_WAVES;   // one CTA per SM
   }
   const bool window = sparse && a->sparsity == B200ATTN_WINDOW;
+  const bool lists = sparse && a->sparsity == B200ATTN_BLOCK_LIST;
+  p.packed = PackedGrid{};
+  // (block lists: a CTA finds its own place, ~1 us on its way, and the longest length is known there)
+  if (a->cu_seqlens && all_rows && a->batch <= kSchedMaxBatch && !lists) {
+    p.packed = packed_grid(a->batch, a->total_tokens, a->heads_q, a->causal || window,
+                           (long long)((kSchedHeads - 1) / p.group + 1) * a->head_dim * 4);
+    // Few items, so that the look-up shows and their order does not matter much, and a grid of batch x longest
+    // that is not mostly empty: that grid (8 heads, 4096 and 1024 tokens, causal 67.9 -> 61.6 us, not causal
+    // 67.6 -> 60.6; 4 x 50-400 x 32 heads, not causal 25.1 -> 21.9).  Equal lengths need no look-up, and keep
+    // the packed order where there are more items than SMs (2 x 2048 x 16 / 4 heads: 47 us in the grid's
+    // order, 36 so; one of 3000 tokens, 8 heads, not causal, 96 items: 49.9 us so, 47.9 in the grid).
+    const bool equal = equal_lengths(a->batch, a->total_tokens, maxlen);
+    const long long items = a->heads_q * packed_tiles_bound(a->batch, a->total_tokens, kPairM, p.n_pairs);
+    if (items <= (equal ? 1LL : 2LL) * p.prefetch_ahead && tight_grid(a->batch, a->total_tokens, kPairM, p.n_pairs))
+      p.packed = PackedGrid{};
+    else if (equal)
+      p.packed.equal = p.n_pairs;
+  }
   p.causal = window ? 1 : (a->causal ? 1 : 0);
   p.window = window ? 1 : 0;
   p.win_local = window ? (a->window_local > (1 << 30) ? (1 << 30) : a->window_local) : 0;
@@ -1143,7 +1162,6 @@ int prefill_fwd(const b200attn_prefill_args* a, bool sparse, cudaStream_t stream
   p.scale_log2 = a->softmax_scale * (a->scale_has_log2e ? 1.f : 1.4426950408889634f);
   p.lse_base2 = a->lse_base2;
   p.status_word = a->status_word;
-  const bool lists = sparse && a->sparsity == B200ATTN_BLOCK_LIST;
   p.block_idx = lists ? a->block_idx : nullptr;
   p.block_cnt = lists ? a->block_cnt : nullptr;
   p.n_qblocks = a->n_qblocks; p.max_nnz = a->max_nnz;

@@ -31,6 +31,7 @@ struct PackedGrid {
   int n_chunks;
   int heads;       // heads scheduled together
   int by_length;   // the weight of a tile is its sequence's length, not its level
+  int equal;       // tiles of every sequence where the host knows that all are of one length, else 0
 };
 
 struct PackedItem {
@@ -45,19 +46,49 @@ inline PackedGrid packed_grid(int batch, long long total_tokens, int heads, bool
   if (seqs < least) seqs = least;
   if (seqs < 1) seqs = 1;
   if (seqs > 32) seqs = 32;
+  if (seqs > batch) seqs = batch;
   PackedGrid g;
   g.seqs = (int)seqs;
   g.n_chunks = (int)((batch + seqs - 1) / seqs);
   const int groups = (heads + kSchedHeads - 1) / kSchedHeads;
   g.heads = (heads + groups - 1) / groups;
   g.by_length = causal ? 0 : 1;
+  g.equal = 0;
   return g;
+}
+
+// All lengths are max_seqlen when they add up to batch x max_seqlen.
+inline bool equal_lengths(int batch, long long total_tokens, int max_seqlen) {
+  return (long long)batch * max_seqlen == total_tokens;
+}
+// Does a grid of batch x tiles of the longest sequence hold few tiles that do not exist (fewer than 3
+// for 4 that may)?  Then a CTA is better off finding its place from its number: looking it up takes
+// about a microsecond, an empty CTA about half of one.
+inline bool tight_grid(int batch, long long total_tokens, int tile, int max_tiles) {
+  return 4LL * batch * max_tiles <= 7 * (total_tokens / tile + batch);
 }
 
 // upper bound on the number of tiles of all sequences (each of them cut at max_tiles tiles)
 inline long long packed_tiles_bound(int batch, long long total_tokens, int tile, int max_tiles) {
   const long long by_total = total_tokens / tile + batch, by_max = (long long)batch * max_tiles;
   return by_total < by_max ? by_total : by_max;
+}
+
+// Item `idx` of a launch of g.equal tiles of every sequence: the order packed_item gives, without a look
+// at the lengths.
+__device__ __forceinline__ void equal_item(const PackedGrid g, int batch, int heads, int idx, PackedItem& out) {
+  const int b0 = idx / (g.seqs * g.equal * heads) * g.seqs;
+  const int n = min(g.seqs, batch - b0);
+  idx -= b0 * g.equal * heads;
+  const int per_group = n * g.equal * g.heads;
+  const int grp = idx / per_group;
+  const int in_grp = idx - grp * per_group;
+  const int g_heads = min(g.heads, heads - grp * g.heads);
+  const int rank = in_grp / g_heads;
+  out.head = grp * g.heads + in_grp - rank * g_heads;
+  out.level = g.equal - 1 - rank / n;
+  out.b = b0 + rank % n;
+  out.n_tiles = g.equal;
 }
 
 // Item `idx` of the launch; false when there are fewer.  Executed by whole converged warps.
