@@ -596,36 +596,48 @@ rmsnorm_bwd_vec_kernel(const XT* __restrict__ dy, const XT* __restrict__ x, cons
   }
 }
 
-// dw[c] = sum of the partial rows' column c, in a fixed order: 32 columns per CTA, a warp per 32nd
+// dw[c] = sum of the partial rows' column c, in a fixed order: 32 columns per CTA, a warp per ROWSth
 // partial row, so that a thread has a handful of independent loads instead of a chain of all rows
 // (148 partial rows of 4096 columns: 14 us with one thread per column).
-constexpr int kDwRows = 32;
-template <typename WT>
-__global__ void __launch_bounds__(32 * kDwRows)
+template <typename WT, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS)
 rmsnorm_dw_reduce_kernel(const float* partial, WT* __restrict__ dw, int D, int n_partial) {
   sm100::grid_dependency_wait();
-  __shared__ float part[kDwRows][33];
+  __shared__ float part[ROWS][33];
   const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (c < D) {
 #pragma unroll 8
-    for (int i = r; i < n_partial; i += kDwRows) s += partial[(long long)i * D + c];
+    for (int i = r; i < n_partial; i += ROWS) s += partial[(long long)i * D + c];
   }
   part[r][lane] = s;
   __syncthreads();
-  // warp r adds the kDwRows sums of column r of this CTA
-  float t = part[lane][r];
+  if constexpr (ROWS == 32) {
+    // warp r adds the sums of column r of this CTA
+    float t = part[lane][r];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  const int cr = blockIdx.x * 32 + r;
-  if (lane == 0 && cr < D) dw[cr] = from_f<WT>(t);
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const int cr = blockIdx.x * 32 + r;
+    if (lane == 0 && cr < D) dw[cr] = from_f<WT>(t);
+  } else if (r == 0 && c < D) {
+    float t = part[0][lane];
+#pragma unroll
+    for (int i = 1; i < ROWS; ++i) t += part[i][lane];
+    dw[c] = from_f<WT>(t);
+  }
 }
 
 template <typename WT>
 cudaError_t launch_dw_reduce(const float* partial, void* dw, int D, int n_partial, cudaStream_t stream) {
-  return launch_after(rmsnorm_dw_reduce_kernel<WT>, dim3((D + 31) / 32), dim3(32 * kDwRows), 0, stream, partial,
-                      (WT*)dw, D, n_partial);
+  auto launch = [&](auto kern, int rows) {
+    return launch_after(kern, dim3((D + 31) / 32), dim3(32 * rows), 0, stream, partial, (WT*)dw, D, n_partial);
+  };
+  // Eight rows a thread at most while that takes few warps: CTAs of 1024 threads start later than there
+  // is to add (whole backward, replayed: one row of 16384 bf16 11.4 -> 10.2 us, 64 rows of 4096 6.8 -> 6.0).
+  if (n_partial <= 32) return launch(rmsnorm_dw_reduce_kernel<WT, 4>, 4);
+  if (n_partial <= 64) return launch(rmsnorm_dw_reduce_kernel<WT, 8>, 8);
+  return launch(rmsnorm_dw_reduce_kernel<WT, 32>, 32);
 }
 
 bool valid_dtypes(int xd, int wd) {
