@@ -52,6 +52,72 @@ def test_packed_schedule_equals_single_sequences(lens, hq, hkv, d):
         assert (dq[:, s].float() - dq1.float()).abs().max() <= 2 ** -7 * dq1.float().abs().max()
 
 
+# More tiles than two to an SM, so that CTAs take over a second and further items: whole and cut tiles in
+# turn, empty sequences between them, both widths the kernel is built for (128: P over S; 64: P beside it)
+# and both that are padded into one of them, causal and not, without and with the longest length; the last
+# three of one length each, in CTAs that take over items and one to a CTA.
+MANY = [256, 1, 0, 255, 257, 700, 128, 511, 30, 513, 384]
+
+
+@pytest.mark.parametrize("lens,h,d,causal", [
+    (MANY, 40, 128, True), (MANY, 40, 64, True), (MANY, 36, 96, False), (MANY, 36, 32, False), (MANY[::-1], 36, 128, False),
+    ([300, 256, 129] * 5, 20, 128, True), ([300, 256, 129] * 5, 20, 64, False), ([300] * 15, 12, 128, True),
+    ([300] * 15, 12, 96, False), ([700] * 5, 12, 64, True),
+])
+def test_taken_over_items_equal_single_sequences(lens, h, d, causal):
+    ops = _ops()
+    q, k, v, _, cu = _packed(lens, h, h // 4, d, torch.bfloat16, seed=2)
+    at = cu.tolist()
+    for kw in ({}, {"max_seqlen": max(lens)}):
+        for _ in range(2):
+            o, lse = ops.prefill(q, k, v, cu_seqlens=cu, causal=causal, **kw)
+            for b, n in enumerate(lens):
+                if n:
+                    s = slice(at[b], at[b + 1])
+                    o1, l1 = ops.prefill(*(t[:, s].contiguous() for t in (q, k, v)), causal=causal)
+                    assert torch.equal(o[:, s], o1) and torch.equal(lse[:, s], l1), (b, n, kw)
+
+
+@pytest.mark.parametrize("lens,causal", [([700, 129, 1, 0, 640], True), ([300] * 7, True), ([300, 256, 129] * 5, False),
+                                         ([900] + [40] * 9, True)])
+def test_backward_with_and_without_the_longest_length(lens, causal):
+    """Handed out on the device, or by the grid of batch x longest where that is given and tight."""
+    ops = _ops()
+    q, k, v, do, cu = _packed(lens, 12, 6, 64, torch.float16, seed=5)
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu, causal=causal)
+    dq, dk, dv = ops.prefill_bwd(q, k, v, o, do, lse, cu_seqlens=cu, causal=causal)
+    dqm, dkm, dvm = ops.prefill_bwd(q, k, v, o, do, lse, cu_seqlens=cu, causal=causal, max_seqlen=max(lens))
+    assert torch.equal(dk, dkm) and torch.equal(dv, dvm)
+    # dq is summed by reduce-adds in arrival order: one rounding of the 16-bit result
+    assert (dq.float() - dqm.float()).abs().max() <= 2 ** -10 * dq.float().abs().max()
+
+
+@pytest.mark.parametrize("d", [128, 64, 32])
+@pytest.mark.parametrize("local,glob", [(64, 0), (100, 200), (1, 130), (0, 64), (300, 5), (0, 0)])
+def test_taken_over_window_items_equal_single_sequences(d, local, glob):
+    """Walks with a gap behind the global prefix, tiles that take no part in some steps, packed and of
+    one length."""
+    ops = _ops()
+    win = dict(sparsity=ops.WINDOW, window_local=local, window_global=glob)
+    lens, h = [700, 129, 1, 0, 513, 256, 900, 300, 64, 1025, 640, 333], 16
+    q, k, v, _, cu = _packed(lens, h, h // 2, d, torch.bfloat16, seed=4)
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu, **win)
+    om, lsem = ops.prefill(q, k, v, cu_seqlens=cu, max_seqlen=max(lens), **win)
+    assert torch.equal(o, om) and torch.equal(lse, lsem)
+    at = cu.tolist()
+    for b, n in enumerate(lens):
+        if n:
+            s = slice(at[b], at[b + 1])
+            o1, l1 = ops.prefill(*(t[:, s].contiguous() for t in (q, k, v)), **win)
+            assert torch.equal(o[:, s], o1) and torch.equal(lse[:, s], l1), (b, n)
+    n, rows = 330, 11
+    q, k, v = (t[:, :n * rows].reshape(rows, n, -1, d) for t in (q, k, v))
+    o, lse = ops.prefill(q, k, v, **win)
+    for b in range(rows):
+        o1, l1 = ops.prefill(*(t[b:b + 1].contiguous() for t in (q, k, v)), **win)
+        assert torch.equal(o[b:b + 1], o1) and torch.equal(lse[b:b + 1], l1), b
+
+
 def test_packed_call_without_lengths_can_be_captured():
     """No length goes back to the host any more: the call fits into a CUDA graph."""
     ops = _ops()
@@ -96,10 +162,41 @@ def test_native_calls_equal_python_calls(monkeypatch):
             out += [y, r, *ops.rmsnorm_bwd(y, xx, w, r)]
         return out
 
+    real, answered = ops._native, {}
+
+    def spy(name, *args):
+        r = real(name, *args)
+        answered.setdefault(name, []).append(r is not None)
+        return r
+    monkeypatch.setattr(ops, "_native", spy)
     native = results()
     n = ops.launch_counter
     ops.prefill(q, k, v, cu_seqlens=cu)
     assert ops.launch_counter == n + 1
+    # who answered: plain arguments are taken natively, the other forms are not
+    take = lambda name, *args, **kw: (answered.clear(), getattr(ops, name)(*args, **kw), answered[name] == [True])[2]
+    idx = torch.zeros(3, 2, 1, dtype=torch.int32, device="cuda")
+    nb = torch.zeros(1, 4, 5, 1, dtype=torch.int32, device="cuda")
+    one = torch.tensor([0, 300], dtype=torch.int32, device="cuda")
+    q1, k1, v1 = (t[:, :300].contiguous() for t in (q[:, :, :4], k, v))
+    pages = kc[:, :256].reshape(12, 64, 2, 128)
+    o, lse = ops.prefill(q, k, v, cu_seqlens=cu)
+    y, r = ops.rmsnorm_fwd(x, w, 1e-6)
+    assert take("prefill", q, k, v, cu_seqlens=cu) and take("prefill", q, k, v)
+    assert take("prefill", wide, k, v, cu_seqlens=cu)           # strided rows the kernels can address
+    assert take("prefill", q, k, v, cu_seqlens=cu, window_local=5, sparsity=ops.WINDOW)
+    assert take("prefill", q1, k1, v1, cu_seqlens=one, max_seqlen=300, sparsity=ops.BLOCK_LIST, block_idx=nb,
+                block_cnt=torch.ones_like(nb[..., 0]))
+    assert take("prefill_bwd", q, k, v, o, do, lse, cu_seqlens=cu)
+    assert take("decode", qd, kc, vc, seqlens=lens) and take("decode", qd, kc, vc, cu_seqlens=cu[:4].contiguous())
+    assert take("decode", qd, kc, vc, seqlens=lens, sparsity=ops.BLOCK_LIST, block_idx=idx)
+    assert take("paged_decode", qd, pages, pages, (table % 12), lens)
+    assert take("append_kv", kc.clone(), vc.clone(), k[0, :3].contiguous(), v[0, :3].contiguous(), lens)
+    assert take("topk_blocks", scores, 7) and take("rmsnorm_fwd", x, w, 1e-6) and take("rmsnorm_bwd", y, x, w, r)
+    assert not take("prefill", odd, k, v, cu_seqlens=cu)        # rows that have to be copied first
+    assert not take("prefill", q, k, v, cu_seqlens=cu.long()) and not take("prefill", q, k, v, cu_seqlens=cu.cpu())
+    assert not take("decode", qd, kc, vc, seqlens=lens.long()) and not take("decode", qd, kc, vc, seqlens=lens.cpu())
+    assert not take("rmsnorm_fwd", x.T, torch.rand(40, device="cuda"), 1e-6)
     monkeypatch.setattr(ops, "_native", lambda *a: None)
     python = results()
     assert len(native) == len(python)
@@ -161,3 +258,36 @@ def test_one_chunk_decoding_equals_split_decoding(d, dtype, lens):
     rep = 40
     big = ops.decode(q.repeat(rep, 1, 1), k.repeat(rep, 1, 1, 1), v.repeat(rep, 1, 1, 1), seqlens=sl.repeat(rep), chunk=64)
     assert torch.equal(big, many.repeat(rep, 1, 1))
+
+
+@pytest.mark.parametrize("d,page", [(128, 16), (128, 64), (64, 64), (96, 48)])
+def test_taken_over_paged_items_equal_a_small_batch(d, page):
+    """More items than fit the chip at once, whole pages that lie in order or not: bit-equal to a batch
+    that takes one item per CTA at the same split."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(7)
+    lens = [1, 0, 1000, 63, 512, 999, 64, 700]
+    B, per, rep = len(lens), -(-1024 // page), 12
+    pool = B * per
+    k, v = (torch.randn(pool, page, 2, d, generator=g, device="cuda").bfloat16() for _ in range(2))
+    table = torch.arange(pool, dtype=torch.int32, device="cuda").view(B, per).clone()
+    table[::2] = table[::2].flip(1)
+    q, sl = torch.randn(B, 8, d, generator=g, device="cuda").bfloat16(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    small = ops.paged_decode(q, k, v, table, sl, chunk=128)
+    big = ops.paged_decode(q.repeat(rep, 1, 1), k, v, table.repeat(rep, 1), sl.repeat(rep), chunk=128)
+    assert torch.equal(big, small.repeat(rep, 1, 1))
+
+
+@pytest.mark.parametrize("glob,local", [(64, 300), (0, 129), (128, 64)])
+@pytest.mark.parametrize("d", [128, 64])
+def test_taken_over_window_decoding_equals_a_small_batch(d, glob, local):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(8)
+    lens, rep = [1, 0, 1000, 63, 512, 999, 130, 700], 24
+    q = torch.randn(len(lens), 8, d, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(len(lens), 1000, 2, d, generator=g, device="cuda").bfloat16() for _ in range(2))
+    sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kw = dict(sparsity=ops.WINDOW, window_global=glob, window_local=local, chunk=64)
+    small = ops.decode(q, k, v, seqlens=sl, **kw)
+    big = ops.decode(q.repeat(rep, 1, 1), k.repeat(rep, 1, 1, 1), v.repeat(rep, 1, 1, 1), seqlens=sl.repeat(rep), **kw)
+    assert torch.equal(big, small.repeat(rep, 1, 1))
