@@ -61,3 +61,19 @@ def test_block_lists_are_split_by_waves(lib, batch, hkv, blocks, want):
     slots, stages, units = 296, blocks, batch * hkv
     cost = lambda c: -(-units * c // slots) * (-(-stages // c) + 3)
     assert cost(n) == min(cost(c) for c in range(1, min(stages, 128) + 1))
+
+
+@pytest.mark.parametrize("batch,hkv,visible,want", [
+    (8, 8, 1024, 1), (8, 8, 2048, 4),        # 64 units: one chunk, then 4 x 64 = 256 items in one wave
+    (12, 8, 4096, 3), (24, 8, 2048, 1),      # 96 x 3 = 288 items, not 384; 192 units in one wave, not two
+    (31, 8, 4096, 1), (16, 8, 32768, 16),    # 248 units in one wave; 2048 keys beyond 8192
+])
+def test_splits_of_a_medium_batch_fill_their_waves(lib, batch, hkv, visible, want):
+    assert _chunks(lib, batch=batch, heads_q=4 * hkv, heads_kv=hkv, max_seqlen=visible) == want
+
+
+def test_short_block_lists_are_not_split(lib):
+    """A second kernel costs more than two or three stages of the first save."""
+    for batch, blocks in [(16, 4), (8, 8)]:
+        assert _chunks(lib, batch=batch, heads_q=32, heads_kv=8, max_seqlen=1 << 20, sparsity=2, block_size=64,
+                       max_sel=blocks) == 1

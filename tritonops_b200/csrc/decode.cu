@@ -22,6 +22,7 @@
 // second (d again) may be permuted freely, which is what lets a thread feed
 // 8 consecutive d of one token row (one 16-byte load) to the instruction:
 // the C fragment of S^T is, register for register, the B fragment of P^T.
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -840,14 +841,21 @@ static int decode_max_visible(const b200attn_decode_args* a) {
 // (two CTAs per SM) and ragged batches need several chunks per CTA to balance.  A unit is a
 // (sequence, KV head, 16 query heads).  Measured on B200 (bf16, D = 128; us of phases 1 and 2):
 //   block lists and windows (every unit has about the same number of keys): the number of chunks
-//     with the least waves x (stages of a chunk + 3), a chunk's fixed cost being ~3 stages.  256
-//     units x 4096 keys: 86.5 in one chunk, 90.6 in two, 93.0 in four; 512 x 2112: 87.4 / 92.4;
-//     16 x 2560: 12.7 in 192-key chunks, 14.2 in 512.
+//     with the least waves x (stages of a chunk + 3), a chunk's fixed cost being ~3 stages, and 6 more
+//     where there is a second kernel.  256 units x 4096 keys: 86.5 in one chunk, 90.6 in two, 93.0 in
+//     four; 512 x 2112: 87.4 / 92.4; 16 x 2560: 12.7 in 192-key chunks, 14.2 in 512; 64 x 512: 12.3 in
+//     one chunk, 14.0 in 128 (with a third of the blocks listed 8.2 / 12.3).
 //   lengths up to max_seqlen, 256 units or more: 2048 keys is best or within 1 % of best (64
 //     sequences x 8 heads, 1024-8192 keys: 187.5; 188.8 at 1024, 194 at 4096).
-//   64 to 255 units: 1024 keys up to 8192, 2048 beyond (192 units, 300-6000 keys in pages of 64: 62.9,
-//     70.6 in one chunk each; 64 units, 200-30000 keys: 87.9, 100 at 8192; 128 units, 2000-16000:
-//     120.7, 135 at 4096, 118.9 at 8192).
+//   64 to 255 units: one chunk up to 1024 keys, 2048 keys beyond 8192, between them of 384 to 4096 keys the
+//     size with the least waves x (stages of a chunk + 4) + a quarter of a chunk (ragged lengths) + 9 where
+//     there is more than one chunk (the second kernel), all lengths taken as max_seqlen.  All lengths that /
+//     an eighth of it to all / all an eighth, replayed: 96 units x 4096 keys 45.0 / 28.1 / 14.4 in 1024-key
+//     chunks, 38.9 / 29.1 / 14.3 in 1536; 192 x 2048: 45.0 / 26.0 / 12.3, 34.8 / 27.6 / 9.2 in one chunk;
+//     64 x 2048: 18.4 / 18.4 / 10.3, 19.0 / 14.9 / 10.9 in 512; 248 x 4096: 88.6 / 65.7 / 18.5, 80.1 / 63.4 /
+//     13.9 in one.  Up to 1024 keys the launch may have fewer CTAs than SMs, but no second kernel: 64 x
+//     1024: 14.8 / 13.3 / 5.6 in one chunk, 13.4 / 12.3 / 8.4 in 384; 96 x 1024: 15.6 / 14.8 / 5.8, 16.4 /
+//     14.9 / 9.2.
 //   fewer: the longest power-of-two chunk that still gives one CTA per SM (8 units x 131072 keys:
 //     5900 GB/s at 4096, 3270 at 512).
 constexpr int kDecodeSlots = 2 * 148;
@@ -865,15 +873,25 @@ static int decode_chunk(const b200attn_decode_args* a) {
     long long best = 1, best_cost = -1;
     for (long long c = 1; c <= stages && c <= 128; ++c) {
       const long long per = (stages + c - 1) / c;
-      const long long cost = ((units * c + kDecodeSlots - 1) / kDecodeSlots) * (per + 3);
+      const long long cost = ((units * c + kDecodeSlots - 1) / kDecodeSlots) * (per + 3) + (c > 1 ? 6 : 0);
       if (best_cost < 0 || cost < best_cost) { best = per; best_cost = cost; }
     }
     return (int)(64 * best);
   }
   if (units >= 256) return 2048;
   if (units >= 64) {
+    int c = visible <= 1024 ? 1024 : 2048;
+    if (visible > 1024 && visible <= 8192) {
+      const int sizes[8] = {384, 512, 768, 1024, 1536, 2048, 3072, 4096};
+      const long long stages = (visible + 63) / 64;
+      long long least = -1;
+      for (int s : sizes) {
+        const long long n = (stages + s / 64 - 1) / (s / 64), per = std::min<long long>(stages, s / 64);
+        const long long cost = 4 * ((units * n + kDecodeSlots - 1) / kDecodeSlots) * (per + 4) + per + (n > 1 ? 36 : 0);
+        if (least < 0 || cost < least || (cost == least && n == 1)) { c = s; least = cost; }
+      }
+    }
     // (no more scratch than the module's fixed array has, where longer chunks avoid that)
-    int c = visible <= 8192 ? 1024 : 2048;
     while (c < 8192 && partial_bytes(a, (visible + c - 1) / c) > (size_t)B200ATTN_NOALLOC_SCRATCH_BYTES) c *= 2;
     return c;
   }
