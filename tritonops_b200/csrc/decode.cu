@@ -592,7 +592,7 @@ decode_split_tma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     __syncwarp();
     if (lane == 0) mbar_arrive(item_empty);
     if (n_tiles == 0) {                    // nothing visible in this chunk
-      if (p.max_chunks == 1 && p.direct_o) {
+      if (p.direct_o) {
         for (int idx = threadIdx.x; idx < heads_here * D; idx += 128) {
           const int g = idx / D, d = idx - g * D;
           ((T*)p.o)[(long long)b * p.o_sb + (long long)(hk * p.group + gg * 16 + g) * p.o_sh + d] = from_float<T>(0.f);
@@ -1021,7 +1021,7 @@ static int launch_decode_tma_d(const b200attn_decode_args* a, const DecodeParams
   if (e != cudaSuccess) return B200ATTN_ERR_CUDA;
   if (p.direct_o) {
     set_launch_count(1);
-    return e == cudaSuccess ? B200ATTN_OK : B200ATTN_ERR_CUDA;
+    return B200ATTN_OK;
   }
   switch (a->head_dim) {
     case 32: e = launch_combine<T, 32>(p, g2, stream); break;
