@@ -65,8 +65,8 @@ def test_block_lists_are_split_by_waves(lib, batch, hkv, blocks, want):
 
 @pytest.mark.parametrize("batch,hkv,visible,want", [
     (8, 8, 1024, 1), (8, 8, 2048, 4),        # 64 units: one chunk, then 4 x 64 = 256 items in one wave
-    (12, 8, 4096, 3), (24, 8, 2048, 1),      # 96 x 3 = 288 items, not 384; 192 units in one wave, not two
-    (31, 8, 4096, 1), (16, 8, 32768, 16),    # 248 units in one wave; 2048 keys beyond 8192
+    (12, 8, 4096, 3), (24, 8, 2048, 3),      # 96 x 3 = 288 items, not 384; 576 items in two waves, not 384
+    (24, 8, 5900, 6), (16, 8, 32768, 16),    # 1024 keys; 2048 beyond 8192
 ])
 def test_splits_of_a_medium_batch_fill_their_waves(lib, batch, hkv, visible, want):
     assert _chunks(lib, batch=batch, heads_q=4 * hkv, heads_kv=hkv, max_seqlen=visible) == want

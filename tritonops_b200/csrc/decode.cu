@@ -847,13 +847,14 @@ static int decode_max_visible(const b200attn_decode_args* a) {
 //     one chunk, 14.0 in 128 (with a third of the blocks listed 8.2 / 12.3).
 //   lengths up to max_seqlen, 256 units or more: 2048 keys is best or within 1 % of best (64
 //     sequences x 8 heads, 1024-8192 keys: 187.5; 188.8 at 1024, 194 at 4096).
-//   64 to 255 units: one chunk up to 1024 keys, 2048 keys beyond 8192, between them of 384 to 4096 keys the
+//   64 to 255 units: one chunk up to 1024 keys, 2048 keys beyond 8192, between them of 384 to 1536 keys the
 //     size with the least waves x (stages of a chunk + 4) + a quarter of a chunk (ragged lengths) + 9 where
 //     there is more than one chunk (the second kernel), all lengths taken as max_seqlen.  All lengths that /
 //     an eighth of it to all / all an eighth, replayed: 96 units x 4096 keys 45.0 / 28.1 / 14.4 in 1024-key
-//     chunks, 38.9 / 29.1 / 14.3 in 1536; 192 x 2048: 45.0 / 26.0 / 12.3, 34.8 / 27.6 / 9.2 in one chunk;
-//     64 x 2048: 18.4 / 18.4 / 10.3, 19.0 / 14.9 / 10.9 in 512; 248 x 4096: 88.6 / 65.7 / 18.5, 80.1 / 63.4 /
-//     13.9 in one.  Up to 1024 keys the launch may have fewer CTAs than SMs, but no second kernel: 64 x
+//     chunks, 38.9 / 29.1 / 14.3 in 1536; 192 x 2048: 45.0 / 26.0 / 12.3, 40.5 / 26.3 / 13.3 in 768; 64 x
+//     2048: 18.4 / 18.4 / 10.3, 19.0 / 14.9 / 10.9 in 512.  (Longer chunks
+//     leave ragged batches an uneven end: 192 units of 300-6000 keys in pages of 64, a call 65.4 in 2048-key
+//     chunks, 62 in 1024.)  Up to 1024 keys the launch may have fewer CTAs than SMs, but no second kernel: 64 x
 //     1024: 14.8 / 13.3 / 5.6 in one chunk, 13.4 / 12.3 / 8.4 in 384; 96 x 1024: 15.6 / 14.8 / 5.8, 16.4 /
 //     14.9 / 9.2.
 //   fewer: the longest power-of-two chunk that still gives one CTA per SM (8 units x 131072 keys:
@@ -882,13 +883,13 @@ static int decode_chunk(const b200attn_decode_args* a) {
   if (units >= 64) {
     int c = visible <= 1024 ? 1024 : 2048;
     if (visible > 1024 && visible <= 8192) {
-      const int sizes[8] = {384, 512, 768, 1024, 1536, 2048, 3072, 4096};
+      const int sizes[5] = {384, 512, 768, 1024, 1536};
       const long long stages = (visible + 63) / 64;
       long long least = -1;
       for (int s : sizes) {
         const long long n = (stages + s / 64 - 1) / (s / 64), per = std::min<long long>(stages, s / 64);
         const long long cost = 4 * ((units * n + kDecodeSlots - 1) / kDecodeSlots) * (per + 4) + per + (n > 1 ? 36 : 0);
-        if (least < 0 || cost < least || (cost == least && n == 1)) { c = s; least = cost; }
+        if (least < 0 || cost < least) { c = s; least = cost; }
       }
     }
     // (no more scratch than the module's fixed array has, where longer chunks avoid that)
